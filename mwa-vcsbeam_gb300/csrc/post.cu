@@ -11,6 +11,7 @@
 //    (v_IDX [s][c][i], 4+4-bit or complex FP64): vmApplyJ_kernel followed by
 //    vmBeamform_kernel (form_beam.cpp:122-371) in one pass.
 #include <cooperative_groups.h>
+#include <type_traits>
 
 #include "vgb_launch.cuh"
 
@@ -436,7 +437,439 @@ int launch_incoh(const uint8_t *data, long long nrows, int ninput, float *incoh,
 
 // ---------------------------------------------------------------------------
 // Beamformer for legacy-layout fine voltages v[s][c][i].
-// A block covers 16 channels x 4 samples = 64 voltage rows, four threads per
+// ---------------------------------------------------------------------------
+// One (tile, sample) of one pointing costs 28 multiply-adds (the two Jones
+// rows times the (Q, P) voltages, the sums, the tile's own power), so the FP32
+// pipe bounds the kernels once the weights are read from registers rather
+// than per sample. Sums are kept for pairs of samples in FP32x2, so one issue
+// slot covers two multiply-adds and half of the slots are left for the loads
+// and the widening of the voltages. One beam of 128 tiles x 128 channels x
+// 10,000 samples of 4+4-bit voltages: 1,060 -> 257 us against the row kernel
+// below (FMA pipe 59 % busy, issue 63 %); three beams of 2,000 samples of
+// complex doubles: 1,440 -> 282 us (shared-memory pipe 60-70 %, the FP64
+// voltages read once instead of once per beam).
+
+// The 8 sums of a pair of samples over a tile: a[0..3] += ex, ey (re, im);
+// a[4..7] += |ex|^2, |ey|^2, ex ey* (re, im). w: the two Jones rows with each
+// value doubled into a pair; nw: minus the imaginary parts of w.
+struct LegacyW {
+    float2 xr0, xi0, xr1, xi1, yr0, yi0, yr1, yi1; // row x: (w00, w01), row y: (w10, w11)
+    float2 nxi0, nxi1, nyi0, nyi1;
+    __device__ __forceinline__ void set(float4 a, float4 b)
+    {
+        xr0 = make_float2(a.x, a.x); xi0 = make_float2(a.y, a.y); xr1 = make_float2(a.z, a.z); xi1 = make_float2(a.w, a.w);
+        yr0 = make_float2(b.x, b.x); yi0 = make_float2(b.y, b.y); yr1 = make_float2(b.z, b.z); yi1 = make_float2(b.w, b.w);
+        nxi0 = make_float2(-a.y, -a.y); nxi1 = make_float2(-a.w, -a.w);
+        nyi0 = make_float2(-b.y, -b.y); nyi1 = make_float2(-b.w, -b.w);
+    }
+};
+
+__device__ __forceinline__ void legacy_pair(float2 (&a)[8], const LegacyW &w, float2 qr, float2 qi, float2 pr, float2 pi)
+{
+    const float2 exr = __ffma2_rn(w.nxi1, pi, __ffma2_rn(w.xr1, pr, __ffma2_rn(w.nxi0, qi, __fmul2_rn(w.xr0, qr))));
+    const float2 exi = __ffma2_rn(w.xi1, pr, __ffma2_rn(w.xr1, pi, __ffma2_rn(w.xi0, qr, __fmul2_rn(w.xr0, qi))));
+    const float2 eyr = __ffma2_rn(w.nyi1, pi, __ffma2_rn(w.yr1, pr, __ffma2_rn(w.nyi0, qi, __fmul2_rn(w.yr0, qr))));
+    const float2 eyi = __ffma2_rn(w.yi1, pr, __ffma2_rn(w.yr1, pi, __ffma2_rn(w.yi0, qr, __fmul2_rn(w.yr0, qi))));
+    const float2 nexr = make_float2(-exr.x, -exr.y);
+    a[0] = padd(a[0], exr);
+    a[1] = padd(a[1], exi);
+    a[2] = padd(a[2], eyr);
+    a[3] = padd(a[3], eyi);
+    a[4] = __ffma2_rn(exr, exr, __ffma2_rn(exi, exi, a[4]));
+    a[5] = __ffma2_rn(eyr, eyr, __ffma2_rn(eyi, eyi, a[5]));
+    a[6] = __ffma2_rn(exr, eyr, __ffma2_rn(exi, eyi, a[6]));
+    a[7] = __ffma2_rn(exi, eyr, __ffma2_rn(nexr, eyi, a[7]));
+}
+
+// Stokes and e of one (pointing, sample, channel) from its 8 sums.
+__device__ __forceinline__ void legacy_store(const LegacyArgs &a, int p, int s, int c, const float (&acc)[8])
+{
+    const float bnXX = acc[0] * acc[0] + acc[1] * acc[1] - acc[4];
+    const float bnYY = acc[2] * acc[2] + acc[3] * acc[3] - acc[5];
+    const float bxr = acc[0] * acc[2] + acc[1] * acc[3] - acc[6];
+    const float bxi = acc[1] * acc[2] - acc[0] * acc[3] - acc[7];
+    float *S = a.S + (((long long)p * a.nsamples + s) * a.nstokes) * a.nchan + c;
+    S[0] = a.invw * (bnXX + bnYY);
+    if (a.nstokes == 4) {
+        S[a.nchan] = a.invw * (bnXX - bnYY);
+        S[2 * a.nchan] = 2.0f * a.invw * bxr;
+        S[3 * a.nchan] = -2.0f * a.invw * bxi;
+    }
+    if (a.e) a.e[((long long)p * a.nsamples + s) * a.nchan + c] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
+// The tiles' (Q, P) input pairs into shared memory, checked against the row.
+__device__ __forceinline__ void legacy_inputs(const LegacyArgs &a, uint32_t *pq)
+{
+    const uint32_t ni = 2u * a.nant;
+    for (int ant = threadIdx.x; ant < a.nant; ant += blockDim.x) {
+        uint32_t iq = __ldg(a.polQ + ant), ip = __ldg(a.polP + ant);
+        if (iq >= ni || ip >= ni) {
+            if (blockIdx.x == 0 && blockIdx.y == 0) atomicOr(a.status, kErrBadInput);
+            iq = ip = 0;
+        }
+        pq[ant] = iq | (ip << 16);
+    }
+}
+
+// 4+4-bit voltages. A block covers 32 channels x kG groups of kS samples; the
+// 8 / kG warps of a group take tiles part, part + 8 / kG, ...: each weight is
+// read once for kS samples. The voltages are staged transposed,
+// [group][input][channel][kS samples] bytes, so that a warp's reads are
+// contiguous and one read brings an input's kS samples; channels are rotated
+// by the input's word so that the staging writes fall on all banks too. The
+// warps' partial sums meet in shared memory, four samples of each group at a
+// time.
+constexpr int kL4C = 32, kLWarps = 8;
+constexpr int kL4Red = kLWarps * 4 * 8 * kL4C; // floats of partial sums
+
+template <int kS, int kG> static size_t legacy4_smem(int nant)
+{
+    return (size_t)2 * nant * kL4C * kS * kG + sizeof(float) * kL4Red + (size_t)nant * 4;
+}
+
+__device__ __forceinline__ uint32_t legacy4_slot(uint32_t i, uint32_t c)
+{
+    return i * kL4C + ((c + 4 * ((i >> 2) & 7)) & (kL4C - 1));
+}
+
+// Four samples' nibbles (bytes x + 8, x = -8 .. 7) as two pairs of floats.
+__device__ __forceinline__ void legacy4_widen(uint32_t u, float2 &a, float2 &b)
+{
+    const float2 bias = make_float2(-8388616.0f, -8388616.0f); // 2^23 + 8
+    a = padd(make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7540)),
+                         __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7541))),
+             bias);
+    b = padd(make_float2(__uint_as_float(__byte_perm(u, 0x4B000000u, 0x7542)),
+                         __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7543))),
+             bias);
+}
+
+template <int kS, int kG> __global__ void __launch_bounds__(256, 2) legacy4_kernel(const LegacyArgs a)
+{
+    constexpr int kParts = kLWarps / kG;
+    using Word = typename std::conditional<kS == 8, uint2, uint32_t>::type; // kS samples of one input
+    extern __shared__ __align__(16) unsigned char lsm[];
+    const int ni = 2 * a.nant, nw = ni / 4;
+    float *red = reinterpret_cast<float *>(lsm);
+    Word *vt = reinterpret_cast<Word *>(red + kL4Red);
+    uint32_t *pq = reinterpret_cast<uint32_t *>(vt + (size_t)kG * ni * kL4C);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c0 = blockIdx.x * kL4C, s0 = blockIdx.y * kS * kG;
+
+    legacy_inputs(a, pq);
+    // stage: lane = (channel 4 warp + lane % 4, word lane / 4 of 8), so 8 lanes
+    // read a whole 32-byte sector of a row
+    for (int g = 0; g < kG; g++) {
+        const int cl = 4 * warp + (lane & 3), c = c0 + cl, sg = s0 + g * kS;
+        const uint32_t *v32 = static_cast<const uint32_t *>(a.v) + ((long long)sg * a.nchan + c) * nw;
+        const long long sstep = (long long)a.nchan * nw;
+        const int ns = c < a.nchan ? min(kS, a.nsamples - sg) : 0;
+        Word *vg = vt + (size_t)g * ni * kL4C;
+        int power[kS];
+#pragma unroll
+        for (int s = 0; s < kS; s++) power[s] = 0;
+#pragma unroll 2
+        for (int wd = lane >> 2; wd < nw; wd += 8) {
+            uint32_t w[kS];
+#pragma unroll
+            for (int s = 0; s < kS; s++) w[s] = s < ns ? __ldg(v32 + s * sstep + wd) : 0u;
+            uint32_t t[kS / 4][4];
+#pragma unroll
+            for (int h = 0; h < kS / 4; h++) { // bytes [sample][input] -> [input][sample]
+                const uint32_t l0 = __byte_perm(w[4 * h], w[4 * h + 1], 0x5140);
+                const uint32_t l1 = __byte_perm(w[4 * h + 2], w[4 * h + 3], 0x5140);
+                const uint32_t h0 = __byte_perm(w[4 * h], w[4 * h + 1], 0x7362);
+                const uint32_t h1 = __byte_perm(w[4 * h + 2], w[4 * h + 3], 0x7362);
+                t[h][0] = __byte_perm(l0, l1, 0x5410);
+                t[h][1] = __byte_perm(l0, l1, 0x7632);
+                t[h][2] = __byte_perm(h0, h1, 0x5410);
+                t[h][3] = __byte_perm(h0, h1, 0x7632);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                if constexpr (kS == 8) vg[legacy4_slot(4 * wd + q, cl)] = make_uint2(t[0][q], t[1][q]);
+                else vg[legacy4_slot(4 * wd + q, cl)] = t[0][q];
+            }
+            if (a.incoh) {
+                // |16 v|^2 of four inputs per product (bytes 16 re, 16 im)
+#pragma unroll
+                for (int s = 0; s < kS; s++) {
+                    const int re = (int)(w[s] & 0xF0F0F0F0u), im = (int)((w[s] << 4) & 0xF0F0F0F0u);
+                    power[s] = __dp4a(im, im, __dp4a(re, re, power[s]));
+                }
+            }
+        }
+        if (a.incoh) {
+#pragma unroll
+            for (int s = 0; s < kS; s++) {
+                for (int o = 4; o < 32; o <<= 1) power[s] += __shfl_xor_sync(0xffffffffu, power[s], o);
+                if (lane < 4 && s < ns) a.incoh[(long long)(sg + s) * a.nchan + c] = (float)(power[s] >> 8);
+            }
+        }
+    }
+    __syncthreads();
+
+    const int c = c0 + lane, part = warp % kParts;
+    const bool live = c < a.nchan;
+    const Word *vg = vt + (size_t)(warp / kParts) * ni * kL4C;
+    for (int p = 0; p < a.npointing; p++) {
+        float2 acc[kS / 2][8];
+#pragma unroll
+        for (int k = 0; k < kS / 2; k++)
+#pragma unroll
+            for (int q = 0; q < 8; q++) acc[k][q] = make_float2(0.f, 0.f);
+        const float4 *Wp = a.W + ((long long)p * a.nant * a.nchan + (live ? c : 0)) * 2;
+        const long long wstep = (long long)a.nchan * 2;
+        float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+        if (part < a.nant) {
+            na = __ldg(Wp + part * wstep);
+            nb = __ldg(Wp + part * wstep + 1);
+        }
+        for (int ant = part; ant < a.nant; ant += kParts) {
+            LegacyW w;
+            w.set(na, nb);
+            if (ant + kParts < a.nant) {
+                na = __ldg(Wp + (ant + kParts) * wstep);
+                nb = __ldg(Wp + (ant + kParts) * wstep + 1);
+            }
+            const uint32_t iqp = pq[ant];
+            const Word bq = vg[legacy4_slot(iqp & 0xFFFFu, lane)], bp = vg[legacy4_slot(iqp >> 16, lane)];
+#pragma unroll
+            for (int h = 0; h < kS / 4; h++) {
+                uint32_t wq, wp;
+                if constexpr (kS == 8) {
+                    wq = h ? bq.y : bq.x;
+                    wp = h ? bp.y : bp.x;
+                } else {
+                    wq = bq;
+                    wp = bp;
+                }
+                float2 qr[2], qi[2], pr[2], pi[2];
+                legacy4_widen(((wq >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u, qr[0], qr[1]);
+                legacy4_widen((wq & 0x0F0F0F0Fu) ^ 0x08080808u, qi[0], qi[1]);
+                legacy4_widen(((wp >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u, pr[0], pr[1]);
+                legacy4_widen((wp & 0x0F0F0F0Fu) ^ 0x08080808u, pi[0], pi[1]);
+#pragma unroll
+                for (int k = 0; k < 2; k++) legacy_pair(acc[2 * h + k], w, qr[k], qi[k], pr[k], pi[k]);
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < kS / 4; h++) {
+            if (h > 0 || p > 0) __syncthreads(); // the previous sums have been read
+#pragma unroll
+            for (int k = 0; k < 2; k++)
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    red[((warp * 4 + 2 * k) * 8 + q) * kL4C + lane] = acc[2 * h + k][q].x;
+                    red[((warp * 4 + 2 * k + 1) * 8 + q) * kL4C + lane] = acc[2 * h + k][q].y;
+                }
+            __syncthreads();
+            // (group, sample of the four) pairs over the warps; with one group
+            // the warps 4 h .. 4 h + 3 take them
+            for (int e = kG == 1 ? warp - 4 * h : warp; e >= 0 && e < 4 * kG; e += kLWarps) {
+                const int g = e / 4, sl = e % 4, s = s0 + g * kS + 4 * h + sl;
+                if (!live || s >= a.nsamples) continue;
+                float sum[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    sum[q] = 0.f;
+#pragma unroll
+                    for (int w = 0; w < kParts; w++) sum[q] += red[(((g * kParts + w) * 4 + sl) * 8 + q) * kL4C + lane];
+                }
+                legacy_store(a, p, s, c, sum);
+            }
+        }
+    }
+}
+
+// (float)d, round to nearest even, in integer operations. `bad` is set where
+// the result is not a normal number (zero, infinities and NaN among them).
+__device__ __forceinline__ float narrow(double d, bool &bad)
+{
+    const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
+    const uint32_t h = 2u * hi - 0x70000000u;                      // sign out, exponent bias 1023 -> 127
+    bad |= h - 0x00200000u >= 0x1FC00000u;                         // FP32 exponent not in 1 .. 254
+    uint32_t u = __funnelshift_l(lo, h >> 1, 3);                   // truncated to 23 bits
+    u += ((lo << 3) | (u & 1u)) > 0x80000000u;                     // above half, or half and odd
+    return __uint_as_float(u | (hi & 0x80000000u));
+}
+
+// A call, so that the conversion instructions are never issued predicated off.
+__device__ __noinline__ float4 narrow4_slow(double x, double y, double z, double w)
+{
+    return make_float4((float)x, (float)y, (float)z, (float)w);
+}
+
+__device__ __forceinline__ float4 narrow4(double x, double y, double z, double w)
+{
+    bool bad = false;
+    const float4 f = make_float4(narrow(x, bad), narrow(y, bad), narrow(z, bad), narrow(w, bad));
+    return bad ? narrow4_slow(x, y, z, w) : f;
+}
+
+// Complex FP64 voltages. A block covers 8 channels x kG groups of kS samples:
+// each row is read from memory once for all pointings and kept as FP32, pairs
+// of samples together; thread = (channel lane % 8, tiles part, part + 32 / kG,
+// ... of its group), and the partial sums of a (sample, channel) meet through
+// shuffles, then shared memory. The voltages are narrowed in integer operations:
+// the conversion instruction issues on the FP64 pipe, 2 per clock per SM here,
+// which takes longer than reading them.
+constexpr int kLdC = 8;
+
+__device__ __forceinline__ float2 shfl2(float2 x, int mask)
+{
+    return make_float2(__shfl_xor_sync(0xffffffffu, x.x, mask), __shfl_xor_sync(0xffffffffu, x.y, mask));
+}
+
+template <int kS, int kG> static size_t legacyd_smem(int nant)
+{
+    return sizeof(float4) * (size_t)(kS / 2) * kG * kLdC * (2 * nant + 1) + sizeof(float) * kLWarps * kS * 8 * kLdC +
+           (size_t)nant * 4;
+}
+
+template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kernel(const LegacyArgs a)
+{
+    constexpr int kGroupWarps = kLWarps / kG, kParts = 4 * kGroupWarps, kPairs = kS / 2, kV = 8 * kPairs;
+    extern __shared__ __align__(16) unsigned char lsm[];
+    const int ni = 2 * a.nant, stride = ni + 1;   // odd: the rows of 8 channels fall on different banks
+    float4 *vt = reinterpret_cast<float4 *>(lsm); // [sample pair][channel][input]: re, re, im, im
+    float *red = reinterpret_cast<float *>(vt + (size_t)kPairs * kG * kLdC * stride); // partial sums
+    uint32_t *pq = reinterpret_cast<uint32_t *>(red + kLWarps * kS * 8 * kLdC);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int c0 = blockIdx.x * kLdC, s0 = blockIdx.y * kS * kG;
+
+    legacy_inputs(a, pq);
+    // warp w stages channel w's rows, two sample pairs in flight
+    if (c0 + warp < a.nchan) {
+        const double2 *v = static_cast<const double2 *>(a.v) + ((long long)s0 * a.nchan + c0 + warp) * ni;
+        const long long sstep = (long long)a.nchan * ni;
+        const int ns = min(kS * kG, a.nsamples - s0);
+        // short rows: 32 / ni of them side by side in the warp
+        const int side = ni < 32 ? 32 / ni : 1, sub = ni < 32 ? lane / ni : 0, i0 = ni < 32 ? lane % ni : lane;
+        constexpr int kFly = kPairs * kG >= 2 ? 2 : 1;
+        for (int k0 = sub; k0 < kPairs * kG && sub < side; k0 += kFly * side)
+#pragma unroll 2
+            for (int i = i0; i < ni; i += 32) {
+                double2 d[kFly][2];
+#pragma unroll
+                for (int k = 0; k < kFly; k++)
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {
+                        const int sl = 2 * (k0 + k * side) + q;
+                        d[k][q] = sl < ns ? __ldcs(v + sl * sstep + i) : make_double2(0.0, 0.0);
+                    }
+#pragma unroll
+                for (int k = 0; k < kFly; k++)
+                    if (k0 + k * side < kPairs * kG)
+                        vt[((k0 + k * side) * kLdC + warp) * stride + i] =
+                            narrow4(d[k][0].x, d[k][1].x, d[k][0].y, d[k][1].y);
+            }
+    }
+    __syncthreads();
+
+    const int cl = lane & (kLdC - 1), c = c0 + cl, group = warp / kGroupWarps;
+    const int part = 4 * (warp % kGroupWarps) + (lane >> 3);
+    const bool live = c < a.nchan;
+    const float4 *vc = vt + (group * kPairs * kLdC + cl) * stride;
+    for (int p = 0; p < a.npointing; p++) {
+        float2 acc[kPairs][8];
+#pragma unroll
+        for (int k = 0; k < kPairs; k++)
+#pragma unroll
+            for (int q = 0; q < 8; q++) acc[k][q] = make_float2(0.f, 0.f);
+        const float4 *Wp = a.W + ((long long)p * a.nant * a.nchan + (live ? c : 0)) * 2;
+        const long long wstep = (long long)a.nchan * 2;
+        float4 na = make_float4(0.f, 0.f, 0.f, 0.f), nb = na;
+        if (part < a.nant) {
+            na = __ldg(Wp + part * wstep);
+            nb = __ldg(Wp + part * wstep + 1);
+        }
+        for (int ant = part; live && ant < a.nant; ant += kParts) {
+            LegacyW w;
+            w.set(na, nb);
+            if (ant + kParts < a.nant) {
+                na = __ldg(Wp + (ant + kParts) * wstep);
+                nb = __ldg(Wp + (ant + kParts) * wstep + 1);
+            }
+            const uint32_t iqp = pq[ant], iq = iqp & 0xFFFFu, ip = iqp >> 16;
+#pragma unroll
+            for (int k = 0; k < kPairs; k++) {
+                const float4 q = vc[k * kLdC * stride + iq], r = vc[k * kLdC * stride + ip];
+                legacy_pair(acc[k], w, make_float2(q.x, q.y), make_float2(q.z, q.w), make_float2(r.x, r.y),
+                            make_float2(r.z, r.w));
+            }
+        }
+        // the four lanes of a channel exchange halves twice: each ends with a
+        // quarter `sel` of the kV pairs of sums, added over the four
+        const bool up = lane & 16, right = lane & 8;
+        float2 half[kV / 2], quarter[kV / 4];
+#pragma unroll
+        for (int j = 0; j < kV / 2; j++) {
+            const float2 lo = acc[j / 8][j % 8], hi = acc[(j + kV / 2) / 8][(j + kV / 2) % 8];
+            half[j] = padd(up ? hi : lo, shfl2(up ? lo : hi, 16));
+        }
+#pragma unroll
+        for (int j = 0; j < kV / 4; j++)
+            quarter[j] = padd(right ? half[j + kV / 4] : half[j], shfl2(right ? half[j] : half[j + kV / 4], 8));
+        if (p > 0) __syncthreads(); // the previous pointing's partial sums have been read
+#pragma unroll
+        for (int j = 0; j < kV / 4; j++) {
+            const int sel = (up ? 2 : 0) + (right ? 1 : 0);
+            red[(((warp * 2 + 0) * (kV / 4) + j) * 4 + sel) * kLdC + cl] = quarter[j].x;
+            red[(((warp * 2 + 1) * (kV / 4) + j) * 4 + sel) * kLdC + cl] = quarter[j].y;
+        }
+        __syncthreads();
+        // thread = (sample, channel)
+        const int sl = tid / kLdC, s = s0 + sl;
+        if (sl < kS * kG && live && s < a.nsamples) {
+            float sum[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const int v = (sl % kS / 2) * 8 + q; // the pair of sums; the sample is its half sl % 2
+                sum[q] = 0.f;
+#pragma unroll
+                for (int w = 0; w < kGroupWarps; w++)
+                    sum[q] += red[((((sl / kS * kGroupWarps + w) * 2 + sl % 2) * (kV / 4) + v % (kV / 4)) * 4 + v / (kV / 4)) * kLdC + cl];
+            }
+            legacy_store(a, p, s, c, sum);
+        }
+    }
+}
+
+// The tile: as many sample groups as leave two (4-bit) or three (FP64) blocks'
+// shared memory per SM, so that small arrays spend less on the partial sums
+// (8 tiles of FP64 voltages, 1,000 samples: 29 us with one group, 15 us with
+// eight, 17 us with the row kernel); where one group of the larger kS leaves
+// room for one block only, the smaller kS (256 tiles of 4+4-bit voltages, 4,000
+// samples: 224 us, row kernel 840 us). Arrays past that (more than 768 tiles of
+// 4+4-bit or 877 of FP64 voltages) take the row kernel.
+struct LegacyTile {
+    void (*kern)(LegacyArgs);
+    size_t smem;
+    int channels, samples;
+};
+
+static LegacyTile legacy_tile(bool int4, int nant)
+{
+    const LegacyTile t4[] = {{legacy4_kernel<8, 8>, legacy4_smem<8, 8>(nant), kL4C, 64},
+                             {legacy4_kernel<8, 4>, legacy4_smem<8, 4>(nant), kL4C, 32},
+                             {legacy4_kernel<8, 2>, legacy4_smem<8, 2>(nant), kL4C, 16},
+                             {legacy4_kernel<8, 1>, legacy4_smem<8, 1>(nant), kL4C, 8},
+                             {legacy4_kernel<4, 1>, legacy4_smem<4, 1>(nant), kL4C, 4}};
+    const LegacyTile td[] = {{legacyd_kernel<4, 8>, legacyd_smem<4, 8>(nant), kLdC, 32},
+                             {legacyd_kernel<4, 4>, legacyd_smem<4, 4>(nant), kLdC, 16},
+                             {legacyd_kernel<4, 2>, legacyd_smem<4, 2>(nant), kLdC, 8},
+                             {legacyd_kernel<4, 1>, legacyd_smem<4, 1>(nant), kLdC, 4},
+                             {legacyd_kernel<2, 1>, legacyd_smem<2, 1>(nant), kLdC, 2}};
+    const LegacyTile *t = int4 ? t4 : td;
+    for (int k = 0; k < 4; k++)
+        if (t[k].smem <= (size_t)(int4 ? 113 : k < 3 ? 75 : 113) * 1024) return t[k];
+    return t[4];
+}
+
+// ---------------------------------------------------------------------------
+// Arrays too large for the tiles above. A block covers 16 channels x 4 samples = 64 voltage rows, four threads per
 // row splitting the tiles (tile = part, part + 4, ...) and combining their
 // sums with two shuffles; the 4+4-bit rows are staged in shared memory with a
 // 4-byte pad (33 KB for 256 tiles, so several blocks share an SM).
@@ -565,6 +998,14 @@ int launch_legacy_beam(const LegacyArgs &a, cudaStream_t st)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: %d inputs do not fit the shared-memory tile", ni);
     if ((a.nsamples + kLS - 1) / kLS > 65535)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: at most %d samples per call", 65535 * kLS);
+    const LegacyTile t = legacy_tile(int4, a.nant);
+    if (t.smem <= 227 * 1024) {
+        const int rc = check_cuda(cudaFuncSetAttribute(t.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem),
+                                  "cudaFuncSetAttribute(legacy tile)");
+        if (rc) return rc;
+        t.kern<<<dim3((a.nchan + t.channels - 1) / t.channels, (a.nsamples + t.samples - 1) / t.samples), 256, t.smem, st>>>(a);
+        return check_launch("legacy beam kernel");
+    }
     dim3 grid((a.nchan + kLC - 1) / kLC, (a.nsamples + kLS - 1) / kLS);
     if (int4) {
         int rc = check_cuda(cudaFuncSetAttribute(legacy_beam_kernel<true>,
