@@ -22,6 +22,7 @@
 //      (form_beam.cpp:298-315) and the incoherent sum; or the PFB-only back
 //      end, which writes the packed legacy-order output (pfb.cpp:316-340).
 // The fine-channel voltages never reach HBM on the beamformer path.
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <map>
@@ -34,7 +35,7 @@
 namespace vgb {
 
 constexpr int kT = 8;                      // spectra per CTA
-constexpr int kG = 4;                      // inputs per step (two tiles) of the PFB-only kernel
+constexpr int kG = 4;                      // inputs per step (two tiles)
 constexpr int kThreads = 256;
 constexpr int kWin = kT + kP - 1;          // frames per input per step
 constexpr int kFrameBytes = kK * 2;        // 256
@@ -48,7 +49,6 @@ template <int G> struct FrontSmemT {
     float2 tw[128];                        // W128 twiddles at fft128_tw_slot(k1, j) (16-byte aligned)
     uint64_t bar[2];
 };
-using FrontSmem = FrontSmemT<kG>;
 static_assert(offsetof(FrontSmemT<4>, tw) % 16 == 0 && offsetof(FrontSmemT<8>, tw) % 16 == 0,
               "twiddles are read 16 bytes at a time");
 
@@ -86,50 +86,6 @@ __device__ __forceinline__ uint32_t issue_frames(const VoltView &vv, int cc, int
     return bytes;
 }
 
-// Producer: warp 0 queues step `it`'s frames (and, when a weight map is
-// given, the two Jones rows of its G/2 tiles, tiles past the last one
-// zero-filled) into stage it & 1, one input per lane (lane G the weights), so
-// the copy set-up costs the warp about one input's worth. Step position
-// it * G + li holds input order[it * G + li] when an order is given, else
-// that input itself.
-template <int G>
-__device__ __forceinline__ void produce(FrontSmemT<G> &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
-                                       const CUtensorMap *wmap, unsigned *status, const int *order = nullptr)
-{
-    const int lane = threadIdx.x & 31;
-    const int s = it & 1;
-    const int w_end = min(m0 + kWin, nspectra + kP - 1);
-    uint32_t total = 0;
-    for (int li = 0; li < G; li++)
-        if (it * G + li < vv.ninputs) total += (w_end - m0) * kFrameBytes;
-    constexpr uint32_t kWBytes = (G / 2) * kK * 16;   // one Jones row of G/2 tiles
-    if (wmap) total += 2 * kWBytes;
-    if (lane == 0) mbar_arrive_expect_tx(&sm.bar[s], total);
-    __syncwarp();
-    uint32_t issued = 0;
-    if (lane < G) {
-        const int pos = it * G + lane;
-        if (pos < vv.ninputs)
-            issued = issue_frames(vv, cc, order ? order[pos] : pos, m0, w_end, sm.stage[s][lane][0], &sm.bar[s],
-                                  status);
-    } else if (lane == G && wmap) {
-        tma_load_5d(sm.wst[s][0][0], wmap, 0, 0, 0, (G / 2) * it, cc, &sm.bar[s]);
-        tma_load_5d(sm.wst[s][1][0], wmap, 0, 1, 0, (G / 2) * it, cc, &sm.bar[s]);
-        issued = 2 * kWBytes;
-    }
-    // lanes 0..G issue copies: a butterfly over the lowest 8 (G = 4) or 16 lanes
-#pragma unroll
-    for (int o = G >= 8 ? 8 : 4; o; o >>= 1) issued += __shfl_xor_sync(0xffffffffu, issued, o);
-    if (lane == 0 && issued != total) {
-        // Some frames were outside the buffers: complete the remaining
-        // transaction count so consumers are not left waiting; the status
-        // word already records the error.
-        asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.bar[s])),
-                     "r"(total - issued)
-                     : "memory");
-    }
-}
-
 // Producer of the beamformer kernel, spread over warps so that no warp
 // carries all of a step's copy set-up (every warp meets at the step's block
 // barriers, where the most loaded one sets the pace): lane 0 of warp li
@@ -139,7 +95,7 @@ __device__ __forceinline__ void produce(FrontSmemT<G> &sm, const VoltView &vv, i
 // outside the buffers (the status word records that). The transaction count
 // may be consumed before it is posted; the phase still cannot complete before
 // warp 0's arrival. Called by every thread after the step's first block
-// barrier, as produce() is.
+// barrier.
 template <int G>
 __device__ __forceinline__ void produce_spread(FrontSmemT<G> &sm, const VoltView &vv, int cc, int it, int m0,
                                               int nspectra, const CUtensorMap *wmap, unsigned *status)
@@ -1011,36 +967,114 @@ __global__ void __launch_bounds__(kWsThreads, 1)
 // ---------------------------------------------------------------------------
 // PFB-only kernel: packed legacy-order output (pfb.cpp:297-343).
 // ---------------------------------------------------------------------------
-template <int kW, bool kFpga, bool kDemote>
-__global__ void __launch_bounds__(kThreads, 2) pack_kernel(const PackArgs a)
+// (double)f in integer operations: the conversion instruction issues on the
+// FP64 pipe, 2 per clock per SM here, which alone would take over half of the
+// kernel's time. `bad` is set for zero, subnormals, infinities and NaN.
+__device__ __forceinline__ double widen_f64(float f, bool &bad)
 {
+    const uint32_t u = __float_as_uint(f);
+    bad |= (u & 0x7FFFFFFFu) - 0x00800000u >= 0x7F000000u;
+    return __hiloint2double((((int)u >> 3) & 0x8FFFFFFF) + 0x38000000, (int)(u << 29));
+}
+
+// A call, so that the conversion instructions are never issued predicated off
+// (they occupy the pipe all the same).
+__device__ __noinline__ double2 widen2_slow(float x, float y) { return make_double2((double)x, (double)y); }
+
+__device__ __forceinline__ double2 widen2(float x, float y)
+{
+    bool bad = false;
+    const double2 d = make_double2(widen_f64(x, bad), widen_f64(y, bad));
+    return bad ? widen2_slow(x, y) : d;
+}
+
+// The rows of an input, 32 bytes off the next input's: the complex-double
+// output reads four inputs' values per half warp.
+constexpr int kPackRows = kT * kFftRow + 4;
+
+template <class Tap> struct PackSmem {
+    char2 stage[kG][kWin][kK];             // TMA destination: frames
+    float2 buf[kG][kPackRows];             // WOLA output -> FFT (in place) -> voltages
+    float2 tw[128];                        // W128 twiddles
+    Tap taps[kP][kK / 2];                  // per (tap, sample pair n0 / 2)
+    uint64_t bar_f;
+    uint32_t tmem;
+};
+static_assert(offsetof(PackSmem<float2>, tw) % 16 == 0 && offsetof(PackSmem<float2>, taps) % 16 == 0, "vector alignment");
+
+// Frames of step `it` into the single stage, input order[it * kG + li] by lane
+// 0 of warp li; lane 0 of warp 0 posts the byte count first.
+template <class Tap>
+__device__ __forceinline__ void pack_frames(PackSmem<Tap> &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
+                                            unsigned *status, const int *order)
+{
+    if ((threadIdx.x & 31) != 0) return;
+    const int warp = threadIdx.x >> 5;
+    if (warp >= kG) return;
+    const int w_end = min(m0 + kWin, nspectra + kP - 1);
+    const uint32_t per_input = (w_end - m0) * kFrameBytes;
+    if (warp == 0) {
+        uint32_t total = 0;
+        for (int li = 0; li < kG; li++)
+            if (it * kG + li < vv.ninputs) total += per_input;
+        mbar_arrive_expect_tx(&sm.bar_f, total);
+    }
+    const int pos = it * kG + warp;
+    if (pos < vv.ninputs) {
+        const uint32_t issued = issue_frames(vv, cc, order[pos], m0, w_end, sm.stage[warp][0], &sm.bar_f, status);
+        if (issued != per_input)
+            asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.bar_f)),
+                         "r"(per_input - issued)
+                         : "memory");
+    }
+}
+
+// The beam kernels' front end at three CTAs per SM (taps from shared memory,
+// frames single-buffered and copied while the step's rows are written out, at
+// most 80 registers; the split sums need 122, two CTAs) and the packing of its
+// rows. kDemote is the 4-bit output. Against two CTAs per SM with taps and
+// held words in registers, every column in one CTA and the instruction's
+// conversions: 10,000 spectra x 256 inputs to 4 bits with int32 sums 1,353 ->
+// 1,107 us (issue 69 %, FMA and ALU pipes 42 %), 4,000 spectra to complex
+// double 787 -> 578 us (shared-memory pipe 69 %, DRAM 50 %: 3.6 TB/s written).
+template <int kW, bool kFpga, bool kDemote>
+__global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kernel(const PackArgs a)
+{
+    using Tap = typename WolaTap<kW>::type;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    FrontSmem &sm = *reinterpret_cast<FrontSmem *>(smem_raw);
+    PackSmem<Tap> &sm = *reinterpret_cast<PackSmem<Tap> *>(smem_raw);
     const int tid = threadIdx.x;
     const int cc = blockIdx.y;
     const int m0 = blockIdx.x * kT;
     const int I = a.vv.ninputs;
-    const int nsteps = (I + kG - 1) / kG;
+    // this CTA's steps: a share of the columns per blockIdx.z
+    const int step0 = blockIdx.z * a.steps_per_cta, nsteps = min((I + kG - 1) / kG, step0 + a.steps_per_cta);
 
     // Inputs are taken in the order of their output columns (inv[col] = the
     // input written there), so each step fills kG adjacent columns of every
     // (spectrum, channel) row: one 4-byte store in the 4-bit mode, 64
     // contiguous bytes in the complex-double mode. The per-input results do
     // not depend on the order.
-    int *inv = reinterpret_cast<int *>(smem_raw + sizeof(FrontSmem));
+    int *inv = reinterpret_cast<int *>(smem_raw + sizeof(PackSmem<Tap>));
     for (int j = tid; j < I; j += kThreads) inv[j] = -1;
     __syncthreads();
     for (int i = tid; i < I; i += kThreads) {
         const int io = __ldg(a.i_idx + i);
         if (io >= 0 && io < I) inv[io] = i;
     }
-    init_front(sm, tid);
-    typename WolaTap<kW>::type tp[kP];
+    init_twiddles(sm.tw, tid);
     const int li = tid >> 6, n0 = 2 * (tid & 63);
-    {
+    if (tid < kK / 2) {
         int hc[2][kP];
         load_taps(a.filter, n0, hc);
-        make_taps<kW, kFpga>(hc, tp);
+        Tap t[kP];
+        make_taps<kW, kFpga>(hc, t);
+#pragma unroll
+        for (int p = 0; p < kP; p++) sm.taps[p][tid] = t[p];
+    }
+    if (tid == 0) {
+        mbar_init(&sm.bar_f, 1);
+        fence_mbar_init();
     }
     __syncthreads();
     // i_idx must be a permutation of the inputs: a column nobody writes means
@@ -1051,29 +1085,51 @@ __global__ void __launch_bounds__(kThreads, 2) pack_kernel(const PackArgs a)
         if (tid == 0) atomicOr(a.status, kErrBadInput);
         return;
     }
-    if (tid < 32) produce(sm, a.vv, cc, 0, m0, a.nspectra, nullptr, a.status, inv);
+    if constexpr (kDemote) {
+        if (tid < 32) {
+            tmem_alloc(&sm.tmem, 32);
+            tmem_relinquish();
+        }
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
+    pack_frames(sm, a.vv, cc, step0, m0, a.nspectra, a.status, inv);
 
-    const bool int4 = (a.flags & VGB_PFB_COMPLEX_INT4) != 0;
     const bool imag_first = (a.flags & VGB_PFB_IMAG_PART_FIRST) != 0;
     const int kp = tid & (kK - 1), mh = tid >> 7;
-    // 4-bit mode with 16-byte stores: the last four steps' words of each of
-    // the thread's spectra, oldest in .x, written together every fourth step
-    uint4 held[kT / 2];
-#pragma unroll
-    for (int mi = 0; mi < kT / 2; mi++) held[mi] = make_uint4(0u, 0u, 0u, 0u);
-    for (int it = 0; it < nsteps; it++) {
-        if (!wait_frames(sm, it, a.status)) {
-            drain(sm, it);
-            return;
+    // 4-bit mode with 16-byte stores: four steps' words of each of the thread's
+    // spectra wait in tensor memory (column 4 (it & 3) + mi of its lane, warps
+    // w and w + 4 at columns 0 and 16) and are written together every fourth
+    // step; as registers they would be spilled
+    const uint32_t theld = kDemote ? sm.tmem + ((uint32_t)(32 * ((tid >> 5) & 3)) << 16) + (uint32_t)(16 * (tid >> 7)) : 0u;
+    int it = step0;
+    for (; it < nsteps; it++) {
+        const int phase = (it - step0) & 1;
+        // step it's frames have landed and every thread has written step it - 1's rows
+        const bool got = mbar_wait_bounded(&sm.bar_f, phase, 1u << 22);
+        if (__syncthreads_or(!got)) {
+            // left early: the copies in flight get a bounded chance to land
+            if (tid == 0) {
+                atomicOr(a.status, kErrWaitTimeout);
+                mbar_wait_bounded(&sm.bar_f, phase, 1u << 20);
+            }
+            break;
         }
-        if (tid < 32 && it + 1 < nsteps) produce(sm, a.vv, cc, it + 1, m0, a.nspectra, nullptr, a.status, inv);
-        wola_step<kW, kFpga>(sm, it & 1, li, n0, tp);
+        {
+            Tap t[kP];
+#pragma unroll
+            for (int p = 0; p < kP; p++) t[p] = sm.taps[p][tid & (kK / 2 - 1)];
+            wola_rows<kW, kFpga>(sm.stage[li][0], reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), n0, t);
+        }
         input_barrier(li);
-        fft_step<kDemote, kFpga>(sm, tid);
+        fft_rows<kDemote, kFpga>(reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), sm.tw, tid & 63);
         __syncthreads();
+        // every WOLA read of the stage is done: the next step's frames may land
+        if (it + 1 < nsteps) pack_frames(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status, inv);
         const int col0 = it * kG;              // the step's first output column
         const int ncol = min(kG, I - col0);
-        if (!int4) {
+        if constexpr (!kDemote) {
             // complex double: four adjacent threads write one (spectrum,
             // channel) row's 64 contiguous bytes, so each warp store fills
             // whole sectors
@@ -1083,42 +1139,64 @@ __global__ void __launch_bounds__(kThreads, 2) pack_kernel(const PackArgs a)
                 const int r = idx & (kG - 1), kc = (idx / kG) % kK, ml = idx / (kG * kK);
                 const int m = m0 + ml;
                 if (r >= ncol || m >= a.nspectra) continue;
-                const float2 v = sm.buf[r * kT + ml][kc];
-                const float hi = imag_first ? v.y : v.x;
-                const float lo = imag_first ? v.x : v.y;
+                const float2 v = sm.buf[r][ml * kFftRow + kc];
                 static_cast<double2 *>(a.out)[cc * a.out_cc + ((long long)m * kK + kc) * I + col0 + r] =
-                    make_double2((double)hi, (double)lo);
+                    imag_first ? widen2(v.y, v.x) : widen2(v.x, v.y);
             }
-            continue;
-        }
+        } else {
+            uint32_t words[kT / 2];
 #pragma unroll
-        for (int mi = 0; mi < kT / 2; mi++) {
-            const int ml = mh + 2 * mi;
-            const int m = m0 + ml;
-            if (m >= a.nspectra) continue;
-            const long long o = cc * a.out_cc + ((long long)m * kK + kp) * I + col0;
-            uint32_t word = 0;
+            for (int mi = 0; mi < kT / 2; mi++) {
+                const int ml = mh + 2 * mi;
+                uint32_t word = 0;
 #pragma unroll
-            for (int r = 0; r < kG; r++) {
-                if (r >= ncol) break;
-                // buf holds (im, re)/K: the reference's default output order
-                const float2 v = sm.buf[r * kT + ml][kp];
-                const float hi = imag_first ? v.y : v.x; // first (high / .x) component
-                const float lo = imag_first ? v.x : v.y;
-                const int h4 = (int)hi & 0xF, l4 = (int)lo & 0xF;
-                const uint32_t b = (uint32_t)((h4 << 4) | l4);
-                if (a.word_stores) word |= b << (8 * r);
-                else static_cast<uint8_t *>(a.out)[o + r] = (uint8_t)b;
+                for (int r = 0; r < kG; r++) {
+                    // buf holds (im, re)/K, whole numbers -8 .. 7: the reference's default output order;
+                    // 1.5 * 2^23 more leaves the number in the low bits
+                    const float2 v = padd(sm.buf[r][ml * kFftRow + kp], make_float2(12582912.f, 12582912.f));
+                    const uint32_t x = __float_as_uint(v.x) & 0xFu, y = __float_as_uint(v.y) & 0xFu;
+                    word |= (imag_first ? (y << 4) | x : (x << 4) | y) << (8 * r);
+                }
+                words[mi] = word;
             }
+            const long long row = ((long long)(m0 + mh) * kK + kp) * I + cc * a.out_cc;
+            uint8_t *out = static_cast<uint8_t *>(a.out) + row + col0; // spectrum m0 + mh; + 2 per mi
+            const long long step = 2LL * kK * I;
             if (a.vec_stores) {
                 // I is a multiple of 16, so the steps come in whole groups of
                 // four and every fourth step completes 16 aligned columns
-                held[mi] = make_uint4(held[mi].y, held[mi].z, held[mi].w, word);
-                if ((it & 3) == 3) *reinterpret_cast<uint4 *>(static_cast<uint8_t *>(a.out) + o - 12) = held[mi];
-            } else if (a.word_stores) {
-                *reinterpret_cast<uint32_t *>(static_cast<uint8_t *>(a.out) + o) = word;
+                __syncwarp(); // the tensor-memory accesses are warp-collective
+                tmem_st4(theld + 4 * (it & 3), words);
+                if ((it & 3) == 3) {
+                    uint32_t h[16];
+                    tmem_wait_st();
+                    tmem_ld16(theld, h);
+#pragma unroll
+                    for (int mi = 0; mi < kT / 2; mi++)
+                        if (m0 + mh + 2 * mi < a.nspectra)
+                            *reinterpret_cast<uint4 *>(out + mi * step - 12) = make_uint4(h[mi], h[4 + mi], h[8 + mi], h[12 + mi]);
+                }
+            } else {
+#pragma unroll
+                for (int mi = 0; mi < kT / 2; mi++) {
+                    if (m0 + mh + 2 * mi >= a.nspectra) continue;
+                    uint8_t *o = out + mi * step;
+                    if (a.word_stores) *reinterpret_cast<uint32_t *>(o) = words[mi];
+                    else
+                        for (int r = 0; r < ncol; r++) o[r] = (uint8_t)(words[mi] >> (8 * r));
+                }
             }
         }
+    }
+    if constexpr (kDemote) {
+        __syncwarp();
+        tmem_wait_st();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        if (tid < 32) tmem_dealloc(sm.tmem, 32);
+    } else if (it < nsteps) {
+        __syncthreads();
     }
 }
 
@@ -1250,12 +1328,23 @@ template <int A, bool B, bool C> struct BeamSel {
 template <int A, bool B, bool C> struct PackSel {
     static int run(const PackArgs &a, dim3 grid, cudaStream_t st)
     {
-        const size_t smem = front_smem<kG>() + sizeof(int) * (size_t)kPackMaxInputs;
+        constexpr size_t base = sizeof(PackSmem<typename WolaTap<A>::type>);
         int rc = check_cuda(cudaFuncSetAttribute(pack_kernel<A, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)smem),
+                                                 (int)(base + sizeof(int) * kPackMaxInputs)),
                             "cudaFuncSetAttribute(pack smem)");
         if (rc) return rc;
-        pack_kernel<A, B, C><<<grid, kThreads, smem, st>>>(a);
+        const size_t smem = base + sizeof(int) * (size_t)a.vv.ninputs;
+        // Each CTA takes a share of the steps (the columns are independent), a
+        // multiple of 4 (16 columns: the 4-bit mode's wide stores), so that the
+        // last wave is a small part: about 12 waves of CTAs, at least 8 steps
+        // each (a CTA's set-up costs about half a step).
+        const int nsteps = (a.vv.ninputs + kG - 1) / kG;
+        const long long want = 12LL * 456, ctas = (long long)grid.x * grid.y;
+        int parts = (int)std::min<long long>((want + ctas - 1) / ctas, std::max(1, nsteps / 8));
+        PackArgs b = a;
+        b.steps_per_cta = ((nsteps + parts - 1) / parts + 3) / 4 * 4;
+        grid.z = (nsteps + b.steps_per_cta - 1) / b.steps_per_cta;
+        pack_kernel<A, B, C><<<grid, kThreads, smem, st>>>(b);
         return check_launch("pack_kernel");
     }
 };

@@ -40,6 +40,7 @@ struct PackArgs {
     unsigned *status;       // kErrBadInput when i_idx is not a permutation of the inputs
     bool word_stores;       // 4-bit mode: out and I allow one aligned 4-byte store per 4 columns
     bool vec_stores;        // ... and one aligned 16-byte store per 16 columns
+    int steps_per_cta;      // set by the launcher: steps (4 columns) each CTA takes
 };
 // Largest input count of the packing PFB (its inverse input map lives in
 // shared memory).
