@@ -189,9 +189,15 @@ int launch_ipfb(const IpfbArgs &a, int njobs, cudaStream_t st)
     return check_launch("ipfb_kernel");
 }
 
-// Advance each job's header template [job][8] by n frames.
-__global__ void vdif_advance_kernel(uint32_t *hdr, int njobs, int n)
+// Advance each job's header template [job][8] by n frames; block x > 0 of a job
+// copies part of its last beam samples for the next second.
+__global__ void vdif_advance_kernel(uint32_t *hdr, int njobs, int n, const float4 *esrc, long long esrc_job, float4 *ehist)
 {
+    if (blockIdx.y > 0) {
+        const int job = blockIdx.x, i = (blockIdx.y - 1) * blockDim.x + threadIdx.x;
+        if (i < kHistFrames * kK) ehist[(long long)job * kHistFrames * kK + i] = esrc[job * esrc_job + i];
+        return;
+    }
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= njobs) return;
     uint32_t *h = hdr + j * 8;
@@ -200,10 +206,13 @@ __global__ void vdif_advance_kernel(uint32_t *hdr, int njobs, int n)
     h[1] = vdif_advanced_word(w0, w1, (uint32_t)n, 1);
 }
 
-int launch_vdif_advance(uint32_t *hdr, int njobs, int nframes, cudaStream_t st)
+int launch_vdif_advance(uint32_t *hdr, int njobs, int nframes, cudaStream_t st, const float4 *esrc, long long esrc_job,
+                        float4 *ehist)
 {
     if (njobs <= 0) return VGB_SUCCESS;
-    vdif_advance_kernel<<<(njobs + 127) / 128, 128, 0, st>>>(hdr, njobs, nframes);
+    // grid x: jobs to copy for, at least as many as the header blocks need
+    const dim3 grid = ehist ? dim3(njobs, 1 + (kHistFrames * kK + 127) / 128) : dim3((njobs + 127) / 128);
+    vdif_advance_kernel<<<grid, 128, 0, st>>>(hdr, njobs, nframes, esrc, esrc_job, ehist);
     return check_launch("vdif_advance_kernel");
 }
 

@@ -1282,7 +1282,7 @@ template <int A, bool B, bool C> struct BeamSel {
     // stream is being captured the cached choice is used if known, else 4.
     static int run(const BeamArgs &a, dim3 grid, cudaStream_t st)
     {
-        if (const int forced = g_pfb_variant.load()) return run_g(a, grid, st, forced);
+        if (const int forced = g_pfb_variant.load()) return a.choose_only ? VGB_SUCCESS : run_g(a, grid, st, forced);
         static std::mutex mu;
         static std::map<std::tuple<int, int, int, int, int, bool, bool>, int> cache;
         const auto key = std::make_tuple((int)grid.x, (int)grid.y, a.vv.ninputs, a.nant, a.nstokes, a.e != nullptr,
@@ -1290,7 +1290,7 @@ template <int A, bool B, bool C> struct BeamSel {
         {
             std::lock_guard<std::mutex> lk(mu);
             auto it = cache.find(key);
-            if (it != cache.end()) return run_g(a, grid, st, it->second);
+            if (it != cache.end()) return a.choose_only ? VGB_SUCCESS : run_g(a, grid, st, it->second);
         }
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         cudaStreamIsCapturing(st, &cs);
@@ -1321,7 +1321,7 @@ template <int A, bool B, bool C> struct BeamSel {
             std::lock_guard<std::mutex> lk(mu);
             cache[key] = pick;
         }
-        return run_g(a, grid, st, pick);
+        return a.choose_only ? VGB_SUCCESS : run_g(a, grid, st, pick);
     }
 };
 
@@ -1386,11 +1386,17 @@ int launch_pack(const PackArgs &a, int ncc, unsigned flags, cudaStream_t st)
 // Gather the last P frames of a second into the compact history layout
 // [cc][input][P][K] char2 that the next second reads (the reference keeps a
 // whole voltage block for this, buffer.c:106-124; only 12 frames are used).
+// The same launch empties the extremes the next second gathers into.
 __global__ void hist_gather_kernel(const char2 *cur, long long cur_block, long long cc_cur, int ninputs,
-                                   int nblocks, char2 *hist, long long cc_hist)
+                                   int nblocks, char2 *hist, long long cc_hist, uint32_t *rstat, long long nstat)
 {
     const int cc = blockIdx.z, i = blockIdx.y;
     const int idx = blockIdx.x * blockDim.x + threadIdx.x; // 16-byte word within the 3072 bytes
+    if (rstat) {
+        const long long nthreads = (long long)gridDim.z * gridDim.y * blockDim.x;
+        for (long long e = ((long long)cc * gridDim.y + i) * blockDim.x + threadIdx.x; e < 3 * nstat; e += nthreads)
+            rstat[e] = e < nstat ? ~0u : 0u;
+    }
     if (idx >= kHistFrames * kK / 8) return;
     const long long last_frame = (long long)nblocks * kFramesPerBlock - kHistFrames;
     const int b = (int)(last_frame / kFramesPerBlock), f = (int)(last_frame % kFramesPerBlock);
@@ -1401,11 +1407,11 @@ __global__ void hist_gather_kernel(const char2 *cur, long long cur_block, long l
 }
 
 int launch_hist_gather(const char2 *cur, long long cur_block, long long cc_cur, int ninputs, int nblocks, int ncc,
-                       char2 *hist, long long cc_hist, cudaStream_t st)
+                       char2 *hist, long long cc_hist, uint32_t *rstat, long long nstat, cudaStream_t st)
 {
     dim3 grid(1, ninputs, ncc);
     hist_gather_kernel<<<grid, kHistFrames * kK / 8, 0, st>>>(cur, cur_block, cc_cur, ninputs, nblocks, hist,
-                                                              cc_hist);
+                                                              cc_hist, rstat, nstat);
     return check_launch("hist_gather_kernel");
 }
 

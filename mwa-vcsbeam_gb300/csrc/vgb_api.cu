@@ -184,7 +184,7 @@ namespace {
 // [ncc][nstokes][128] each, or NULL).
 int beamform_mwax_impl(const vgb_voltages *v, int ncc, int nspectra, const int32_t *filter, int ntaps, int nchan,
                        unsigned pfb_flags, const void *W, int nant, float invw, int nstokes, float *S_, void *e,
-                       float *incoh, uint32_t *rstat, void *stream)
+                       float *incoh, uint32_t *rstat, void *stream, bool choose_only = false)
 {
     int rc = check_geometry(ntaps, nchan);
     if (rc) return rc;
@@ -209,6 +209,7 @@ int beamform_mwax_impl(const vgb_voltages *v, int ncc, int nspectra, const int32
     a.e_cc = (long long)nspectra * kK;
     a.incoh = incoh;
     a.inc_cc = (long long)nspectra * kK;
+    a.choose_only = choose_only;
     a.status = status_word();
     if (!a.status) return set_error(VGB_ERR_CUDA, "device status word unavailable");
     if (rstat) {
@@ -460,6 +461,10 @@ struct vgb_pipeline {
     long long second_bytes = 0;      // one coarse channel's second, bytes
     unsigned wola_flags = 0;         // VGB_WOLA_FP32 / VGB_WOLA_FP32_SPLIT for the loaded filter
     cudaStream_t s_comp = nullptr, s_copy = nullptr;
+    // the second's stages that do not depend on one another run beside s_comp:
+    // [0] incoherent renormalise, [1] inverse PFB, [2] voltage history
+    cudaStream_t s_side[3] = {};
+    cudaEvent_t ev_begin = nullptr, ev_beam = nullptr, ev_side[3] = {};
     cudaEvent_t ev_copied[2] = {}, ev_consumed[2] = {};
     int32_t *d_filter = nullptr;
     float *d_coeffs = nullptr;
@@ -476,7 +481,7 @@ struct vgb_pipeline {
     float *d_ioff = nullptr, *d_iscl = nullptr; // [ncc][128]
     uint8_t *d_vdif = nullptr;       // [cc][ns][544]
     uint32_t *d_hdr = nullptr;
-    uint32_t *d_rstat = nullptr;     // [3][cc][stokes][128]: Stokes min / max keys, first-value NaN flags
+    uint32_t *d_rstat[2] = {};       // by second parity: [3][cc][stokes][128] Stokes min / max keys, first-value NaN flags
     long long second = 0;            // seconds completed
     int launches = 0;
     int host_buf = 0;
@@ -547,17 +552,38 @@ vgb_voltages pipeline_voltages(const vgb_pipeline *p, const char2 *volt, long lo
     return v;
 }
 
-// Empty extremes (min keys all ones, max keys and NaN flags zero) for the
-// next second's beam kernel to gather into.
+// Empty extremes (min keys all ones, max keys and NaN flags zero) in both
+// buffers; afterwards every second's history kernel empties the next second's.
 int reset_rstat(vgb_pipeline *p)
 {
     const size_t n = (size_t)p->cfg.ncc * p->cfg.nstokes * kK;
-    int rc = check_cuda(cudaMemsetAsync(p->d_rstat, 0xFF, n * sizeof(uint32_t), p->s_comp), "reset extremes");
-    return rc ? rc : check_cuda(cudaMemsetAsync(p->d_rstat + n, 0, 2 * n * sizeof(uint32_t), p->s_comp),
-                                "reset extremes");
+    int rc = VGB_SUCCESS;
+    for (int b = 0; b < 2 && !rc; b++) {
+        rc = check_cuda(cudaMemsetAsync(p->d_rstat[b], 0xFF, n * sizeof(uint32_t), p->s_comp), "reset extremes");
+        if (!rc)
+            rc = check_cuda(cudaMemsetAsync(p->d_rstat[b] + n, 0, 2 * n * sizeof(uint32_t), p->s_comp), "reset extremes");
+    }
+    return rc;
 }
 
-// One second of compute on s_comp with the voltages at `volt`.
+// Let side stream i start after what s_comp holds now (recorded in `ev`).
+int fork_side(vgb_pipeline *p, cudaEvent_t ev, int i)
+{
+    return check_cuda(cudaStreamWaitEvent(p->s_side[i], ev, 0), "cudaStreamWaitEvent");
+}
+
+int join_side(vgb_pipeline *p, int i)
+{
+    const int rc = check_cuda(cudaEventRecord(p->ev_side[i], p->s_side[i]), "cudaEventRecord");
+    return rc ? rc : check_cuda(cudaStreamWaitEvent(p->s_comp, p->ev_side[i], 0), "cudaStreamWaitEvent");
+}
+
+// One second of compute with the voltages at `volt`, complete on s_comp. The
+// voltage history runs beside the beam kernel, and the two renormalises and the
+// inverse PFB beside one another after it: for one coarse channel each fills the
+// GPU only in part (a second of one channel 1,209 -> 1,158 us, of the smallest
+// array 84 -> 69 us, the full band unchanged). With stage timing on, all in
+// order on s_comp.
 int pipeline_second(vgb_pipeline *p, const char2 *volt, long long cc_stride_bytes)
 {
     NvtxRange range("vgb: pipeline second");
@@ -567,9 +593,25 @@ int pipeline_second(vgb_pipeline *p, const char2 *volt, long long cc_stride_byte
     p->launches = 0;
     const vgb_voltages v = pipeline_voltages(p, volt, cc_stride_bytes);
     const unsigned flags = pipeline_pfb_flags(p);
+    const bool sides = !p->timing;
+    cudaStream_t s_inc = sides ? p->s_side[0] : p->s_comp, s_inv = sides ? p->s_side[1] : p->s_comp;
+    cudaStream_t s_hist = sides ? p->s_side[2] : p->s_comp;
     auto mark = [&](int i) {
         return p->timing ? check_cuda(cudaEventRecord(p->ev_stage[i], p->s_comp), "stage event") : VGB_SUCCESS;
     };
+    // carry the last 12 voltage frames of each input, and empty the next second's extremes
+    auto history = [&]() {
+        p->launches++;
+        return launch_hist_gather(volt, (long long)p->ninputs * kVSPVB, cc_stride_bytes / 2, p->ninputs, c.nblocks, c.ncc,
+                                  p->d_hist[nxt], (long long)p->ninputs * kHistFrames * kK, p->d_rstat[nxt],
+                                  (long long)c.ncc * c.nstokes * kK, s_hist);
+    };
+    if (sides) {
+        rc = check_cuda(cudaEventRecord(p->ev_begin, p->s_comp), "cudaEventRecord");
+        rc = rc ? rc : fork_side(p, p->ev_begin, 2);
+        rc = rc ? rc : history();
+        if (rc) return rc;
+    }
     if ((rc = mark(5))) return rc;
     if (p->tracking) {
         // the second's pointing, B at each coarse channel's beam frequency,
@@ -589,50 +631,51 @@ int pipeline_second(vgb_pipeline *p, const char2 *volt, long long cc_stride_byte
     }
     if ((rc = mark(0))) return rc;
     rc = beamform_mwax_impl(&v, c.ncc, p->nspectra, p->d_filter, kP, kK, flags, p->d_W, c.nant, c.invw, c.nstokes,
-                            p->d_S, p->d_e, p->d_incoh, p->d_rstat, p->s_comp);
+                            p->d_S, p->d_e, p->d_incoh, p->d_rstat[cur], p->s_comp);
     if (rc) return rc;
     p->launches++;
     if ((rc = mark(1))) return rc;
+    if (sides) {
+        rc = check_cuda(cudaEventRecord(p->ev_beam, p->s_comp), "cudaEventRecord");
+        rc = rc ? rc : fork_side(p, p->ev_beam, 0);
+        if (!rc && c.do_ipfb) rc = fork_side(p, p->ev_beam, 1);
+        if (rc) return rc;
+    }
     // spliced PSRFITS rows: [s][st][cc*128 + c]
     const long long row = (long long)c.nstokes * c.ncc * kK;
     rc = renormalise_impl(p->d_S, c.ncc, 1, p->nspectra, c.nstokes, kK, p->d_psrfits, kK, 0, row,
-                          (long long)c.ncc * kK, p->d_off, p->d_scl, p->d_rstat, p->s_comp);
+                          (long long)c.ncc * kK, p->d_off, p->d_scl, p->d_rstat[cur], p->s_comp);
     if (rc) return rc;
     p->launches++;
     // the incoherent beam's 8-bit rows (Stokes I, spliced the same way; its
     // renormalise as cu_form_incoh_beam's, form_beam.cpp:495-497)
     rc = renormalise_impl(p->d_incoh, c.ncc, 1, p->nspectra, 1, kK, p->d_ipsr, kK, 0, (long long)c.ncc * kK,
-                          (long long)c.ncc * kK, p->d_ioff, p->d_iscl, nullptr, p->s_comp);
+                          (long long)c.ncc * kK, p->d_ioff, p->d_iscl, nullptr, s_inc);
     if (rc) return rc;
     p->launches++;
-    // the next second's extremes start empty
-    rc = reset_rstat(p);
-    if (rc) return rc;
     if ((rc = mark(2))) return rc;
     if (c.do_ipfb) {
         const long long ejob = (long long)p->nspectra * kK * 16;
         rc = vgb_ipfb(p->d_e, ejob, p->second > 0 ? p->d_ehist[cur] : nullptr, (long long)kHistFrames * kK * 16,
-                      p->d_coeffs, kP, kK, p->nspectra, c.ncc, nullptr, p->d_vdif, p->d_hdr, 0, p->s_comp);
+                      p->d_coeffs, kP, kK, p->nspectra, c.ncc, nullptr, p->d_vdif, p->d_hdr, 0, s_inv);
         if (rc) return rc;
         p->launches++;
-        // the next second's headers start where this second's end
-        rc = launch_vdif_advance(p->d_hdr, c.ncc, p->nspectra, p->s_comp);
+        // the next second's headers start where this second's end, and the
+        // last 12 beam samples of each coarse channel are carried
+        rc = launch_vdif_advance(p->d_hdr, c.ncc, p->nspectra, s_inv, p->d_e + (long long)(p->nspectra - kHistFrames) * kK,
+                                 (long long)p->nspectra * kK, p->d_ehist[nxt]);
         if (rc) return rc;
         p->launches++;
-        // carry the last 12 beam samples of each coarse channel
-        rc = check_cuda(cudaMemcpy2DAsync(p->d_ehist[nxt], (size_t)kHistFrames * kK * 16,
-                                          p->d_e + (long long)(p->nspectra - kHistFrames) * kK, (size_t)ejob,
-                                          (size_t)kHistFrames * kK * 16, c.ncc, cudaMemcpyDeviceToDevice,
-                                          p->s_comp),
-                        "carry beam history");
-        if (rc) return rc;
     }
     if ((rc = mark(3))) return rc;
-    // carry the last 12 voltage frames of each input
-    rc = launch_hist_gather(volt, (long long)p->ninputs * kVSPVB, cc_stride_bytes / 2, p->ninputs, c.nblocks, c.ncc,
-                            p->d_hist[nxt], (long long)p->ninputs * kHistFrames * kK, p->s_comp);
+    if (sides) {
+        rc = join_side(p, 0);
+        if (!rc && c.do_ipfb) rc = join_side(p, 1);
+        rc = rc ? rc : join_side(p, 2);
+    } else {
+        rc = history();
+    }
     if (rc) return rc;
-    p->launches++;
     if ((rc = mark(4))) return rc;
     p->second++;
     // asynchronous copies of the products into the caller's host buffers
@@ -693,16 +736,15 @@ int pipeline_second_graph(vgb_pipeline *p, const char2 *volt, long long cc_strid
         }
     if (p->graphs.size() >= 8) drop_graphs(p);
     const long long saved = p->second;
-    // one eager fused PFB + beamformer pass first, so the front end's
-    // inputs-per-step choice is timed (and cached) outside the capture; it
-    // writes only the Stokes and beam buffers the second then rewrites
+    // the front end's kernel variant for this shape is timed outside the
+    // capture, if it is not known yet (the timing launches write only the
+    // Stokes and beam buffers the second then rewrites)
     int rc = VGB_SUCCESS;
     if (!p->front_timed) {
         const vgb_pipeline_config &c = p->cfg;
         const vgb_voltages v = pipeline_voltages(p, volt, cc_stride_bytes);
-        rc = vgb_beamform_mwax(&v, c.ncc, p->nspectra, p->d_filter, kP, kK,
-                               pipeline_pfb_flags(p), p->d_W, c.nant, c.invw, c.nstokes,
-                               p->d_S, p->d_e, p->d_incoh, p->s_comp);
+        rc = beamform_mwax_impl(&v, c.ncc, p->nspectra, p->d_filter, kP, kK, pipeline_pfb_flags(p), p->d_W, c.nant, c.invw,
+                                c.nstokes, p->d_S, p->d_e, p->d_incoh, nullptr, p->s_comp, true);
         if (rc) return rc;
         p->front_timed = true; // one shape per pipeline
     }
@@ -742,6 +784,12 @@ int vgb_pipeline_create(const vgb_pipeline_config *cfg, vgb_pipeline **out)
     rc = rc ? rc : check_cuda(cudaStreamCreateWithFlags(&p->s_comp, cudaStreamNonBlocking), "stream");
     rc = rc ? rc : check_cuda(cudaStreamCreateWithFlags(&p->s_copy, cudaStreamNonBlocking), "stream");
     for (int i = 0; i < 6 && !rc; i++) rc = check_cuda(cudaEventCreate(&p->ev_stage[i]), "event");
+    for (int i = 0; i < 3 && !rc; i++) {
+        rc = check_cuda(cudaStreamCreateWithFlags(&p->s_side[i], cudaStreamNonBlocking), "stream");
+        rc = rc ? rc : check_cuda(cudaEventCreateWithFlags(&p->ev_side[i], cudaEventDisableTiming), "event");
+    }
+    rc = rc ? rc : check_cuda(cudaEventCreateWithFlags(&p->ev_begin, cudaEventDisableTiming), "event");
+    rc = rc ? rc : check_cuda(cudaEventCreateWithFlags(&p->ev_beam, cudaEventDisableTiming), "event");
     for (int b = 0; b < 2 && !rc; b++) {
         rc = check_cuda(cudaEventCreateWithFlags(&p->ev_copied[b], cudaEventDisableTiming), "event");
         rc = rc ? rc : check_cuda(cudaEventCreateWithFlags(&p->ev_consumed[b], cudaEventDisableTiming), "event");
@@ -764,7 +812,7 @@ int vgb_pipeline_create(const vgb_pipeline_config *cfg, vgb_pipeline **out)
     rc = rc ? rc : dalloc(&p->d_scl, sizeof(float) * ncc * cfg->nstokes * kK);
     if (cfg->do_ipfb) rc = rc ? rc : dalloc(&p->d_vdif, (size_t)ncc * ns * 544);
     rc = rc ? rc : dalloc(&p->d_hdr, sizeof(uint32_t) * 8 * ncc);
-    rc = rc ? rc : dalloc(&p->d_rstat, sizeof(uint32_t) * 3 * ncc * cfg->nstokes * kK);
+    for (int b = 0; b < 2; b++) rc = rc ? rc : dalloc(&p->d_rstat[b], sizeof(uint32_t) * 3 * ncc * cfg->nstokes * kK);
     rc = rc ? rc : dalloc(&p->d_trk_counter, sizeof(long long));
     rc = rc ? rc : dalloc(&p->d_trk_cur, sizeof(double) * 8);
     rc = rc ? rc : dalloc(&p->d_trk_B, sizeof(double2) * 4 * ncc * cfg->nant);
@@ -797,10 +845,12 @@ int vgb_pipeline_destroy(vgb_pipeline *p)
     if (!p) return VGB_SUCCESS;
     if (p->s_comp) cudaStreamSynchronize(p->s_comp);
     if (p->s_copy) cudaStreamSynchronize(p->s_copy);
+    for (int i = 0; i < 3; i++)
+        if (p->s_side[i]) cudaStreamSynchronize(p->s_side[i]);
     drop_graphs(p);
     void *bufs[] = {p->d_filter, p->d_coeffs, p->d_W, p->d_volt[0], p->d_volt[1], p->d_hist[0], p->d_hist[1],
                     p->d_S, p->d_e, p->d_incoh, p->d_ehist[0], p->d_ehist[1], p->d_psrfits, p->d_off, p->d_scl,
-                    p->d_vdif, p->d_hdr, p->d_rstat, p->d_trk_counter, p->d_trk_cur, p->d_trk_B,
+                    p->d_vdif, p->d_hdr, p->d_rstat[0], p->d_rstat[1], p->d_trk_counter, p->d_trk_cur, p->d_trk_B,
                     p->d_trk_scratch, p->d_ipsr, p->d_ioff, p->d_iscl};
     for (void *b : bufs)
         if (b) cudaFree(b);
@@ -810,6 +860,12 @@ int vgb_pipeline_destroy(vgb_pipeline *p)
         if (p->ev_copied[b]) cudaEventDestroy(p->ev_copied[b]);
         if (p->ev_consumed[b]) cudaEventDestroy(p->ev_consumed[b]);
     }
+    for (int i = 0; i < 3; i++) {
+        if (p->s_side[i]) cudaStreamDestroy(p->s_side[i]);
+        if (p->ev_side[i]) cudaEventDestroy(p->ev_side[i]);
+    }
+    if (p->ev_begin) cudaEventDestroy(p->ev_begin);
+    if (p->ev_beam) cudaEventDestroy(p->ev_beam);
     if (p->s_comp) cudaStreamDestroy(p->s_comp);
     if (p->s_copy) cudaStreamDestroy(p->s_copy);
     delete p;
@@ -959,6 +1015,7 @@ int vgb_pipeline_load_state(vgb_pipeline *p, const void *host, long long bytes)
     if (!rc)
         rc = check_cuda(cudaMemcpy(p->d_trk_counter, &h.second, sizeof(long long), cudaMemcpyHostToDevice),
                         "load tracking counter");
+    if (!rc) rc = reset_rstat(p); // the loaded second's parity may be the other one
     return rc;
 }
 

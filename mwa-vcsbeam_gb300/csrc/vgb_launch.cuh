@@ -27,6 +27,9 @@ struct BeamArgs {
     // whether spectrum 0's value is NaN: [cc][nstokes][K] each (the index of
     // the 8-bit stage's offsets for one pointing)
     uint32_t *st_mn, *st_mx, *st_nan0;
+    // only make sure the kernel variant of this shape is chosen (launches
+    // nothing where it is known already)
+    bool choose_only;
 };
 
 struct PackArgs {
@@ -95,7 +98,9 @@ int launch_beam(const BeamArgs &a, int ncc, unsigned flags, cudaStream_t st);
 // VDIF frames per second (the MWA fine sample rate, 1.28 MHz / 128): where a
 // header's frame number rolls over to the next second.
 constexpr int kVdifFramesPerSecond = 10000;
-int launch_vdif_advance(uint32_t *hdr, int njobs, int nframes, cudaStream_t st);
+// ehist (nullable): also copy each job's kHistFrames beam samples from esrc + job * esrc_job.
+int launch_vdif_advance(uint32_t *hdr, int njobs, int nframes, cudaStream_t st, const float4 *esrc = nullptr,
+                        long long esrc_job = 0, float4 *ehist = nullptr);
 // Force the fused front end's inputs per step (4 or 8), or 0 for the timed
 // choice; returns the previous setting, -1 for a bad value.
 int pfb_variant_last();
@@ -122,8 +127,9 @@ int launch_ipfb(const IpfbArgs &a, int njobs, cudaStream_t st);
 int launch_wola_staged(const VoltView &vv, const int *filter, int nspectra, int2 *b, cudaStream_t st);
 int launch_round_staged(int *data, long long n, int fpga, cudaStream_t st);
 int launch_fft_staged(float2 *rows, long long nrows, cudaStream_t st);
+// rstat: extremes to empty ([3][nstat]: min keys, max keys, NaN flags).
 int launch_hist_gather(const char2 *cur, long long cur_block, long long cc_cur, int ninputs, int nblocks, int ncc,
-                       char2 *hist, long long cc_hist, cudaStream_t st);
+                       char2 *hist, long long cc_hist, uint32_t *rstat, long long nstat, cudaStream_t st);
 struct PbArgs { // primary-beam model evaluation
     const double *az, *za;       // [npointing] radians
     int npointing;
