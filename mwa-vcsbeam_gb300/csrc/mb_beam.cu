@@ -1209,7 +1209,7 @@ constexpr int kRnT = 128; // integrations per transpose chunk
 // memory and writes 16-byte runs of channels.
 __global__ void __launch_bounds__(256, 4) mb_renorm_kernel(const MbRenormArgs a)
 {
-    __shared__ float s_off[32], s_scl[32];
+    __shared__ __align__(16) float s_off[32], s_scl[32];
     __shared__ uint32_t tile[kRnT][9];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int c0 = blockIdx.x * 32;
@@ -1238,15 +1238,13 @@ __global__ void __launch_bounds__(256, 4) mb_renorm_kernel(const MbRenormArgs a)
     __syncthreads();
     // warp w: channels 4w .. 4w+3 of the block
     const float *rows[4];
-    float off[4], scl[4], rcp[4];
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         const int c = c0 + 4 * wid + k;
         rows[k] = a.S + (((long long)(c < a.nfine ? c : c0) * a.B + p) * a.nst + st) * a.nint;
-        off[k] = s_off[4 * wid + k];
-        scl[k] = s_scl[4 * wid + k];
-        rcp[k] = 1.f / scl[k];
     }
+    const float4 off = *reinterpret_cast<const float4 *>(&s_off[4 * wid]), scl = *reinterpret_cast<const float4 *>(&s_scl[4 * wid]);
+    const float4 rcp = make_float4(1.f / scl.x, 1.f / scl.y, 1.f / scl.z, 1.f / scl.w);
     const bool wide = ((a.out_s | a.out_st | a.out_p) & 15) == 0 &&
                       (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && c0 + 32 <= a.nfine;
     for (int t0 = 0; t0 < a.nint; t0 += kRnT) {
@@ -1259,10 +1257,7 @@ __global__ void __launch_bounds__(256, 4) mb_renorm_kernel(const MbRenormArgs a)
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            uint32_t w = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) w |= (uint32_t)quant_u8(e[j][k], off[k], scl[k], rcp[k]) << (8 * k);
-            tile[lane + 32 * j][wid] = w;
+            tile[lane + 32 * j][wid] = quant4_u8(make_float4(e[j][0], e[j][1], e[j][2], e[j][3]), off, scl, rcp);
         }
         __syncthreads();
         const int tl = threadIdx.x >> 1, h = threadIdx.x & 1, t = t0 + tl;

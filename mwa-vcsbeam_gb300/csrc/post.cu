@@ -10,8 +10,10 @@
 //  * beamformer for fine-channel voltages already in legacy layout
 //    (v_IDX [s][c][i], 4+4-bit or complex FP64): vmApplyJ_kernel followed by
 //    vmBeamform_kernel (form_beam.cpp:122-371) in one pass.
-#include <cooperative_groups.h>
+#include <algorithm>
 #include <type_traits>
+
+#include <cooperative_groups.h>
 
 #include "vgb_launch.cuh"
 
@@ -397,9 +399,180 @@ __global__ void __launch_bounds__(256) renorm_kernel(const RenormArgs a)
     }
 }
 
+// Four adjacent channels per thread (16-byte reads, 4-byte writes), for Stokes
+// and bytes aligned to that. A block takes kCh channels of one (cc, pointing,
+// stokes) and a share of the samples.
+//
+// kStats: the extremes come from the beam kernel and a block reads its samples
+// once (a second of one channel 38 -> 12 us). Otherwise a cluster of
+// kRenormSplit blocks covers the samples, each keeps its share in shared memory
+// (asynchronous copies, all in flight at once), the extremes meet through
+// distributed shared memory and the bytes are formed from there, so the Stokes
+// are read from memory once (six beams' second, 123 MB: 76 -> 54 us, now bound
+// by the latencies between the phases; the incoherent beam's second of one
+// channel 37 -> 9.5 us). kCh is the largest of 32, 16 and 8 whose share leaves
+// five blocks per SM: with 100 KB and two the six beams took 71 us. The scan's
+// semantics are renorm_kernel's, which serves the rest.
+constexpr int kRenormTile = 44 * 1024; // bytes of samples a block may keep: five blocks per SM
+
+__device__ __forceinline__ float4 min4(float4 a, float4 b)
+{
+    return make_float4(fminf(a.x, b.x), fminf(a.y, b.y), fminf(a.z, b.z), fminf(a.w, b.w));
+}
+__device__ __forceinline__ float4 max4(float4 a, float4 b)
+{
+    return make_float4(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z), fmaxf(a.w, b.w));
+}
+__device__ __forceinline__ float4 shfl4(float4 v, int o)
+{
+    return make_float4(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o),
+                       __shfl_xor_sync(0xffffffffu, v.z, o), __shfl_xor_sync(0xffffffffu, v.w, o));
+}
+
+template <int kCh, bool kStats> __global__ void __launch_bounds__(256, 5) renorm4_kernel(const RenormArgs a)
+{
+    namespace cg = cooperative_groups;
+    constexpr int kThr = 256, kQ = kCh / 4, kRows = kThr / kQ; // threads per row, rows per pass
+    extern __shared__ __align__(16) float4 rsm[];
+    __shared__ float4 smin[kThr / 32][kQ], smax[kThr / 32][kQ];
+    __shared__ __align__(16) float s_par[3][kCh]; // offset, scale, 1 / scale
+    const int tid = threadIdx.x, q = tid % kQ, row = tid / kQ;
+    const int nparts = kStats ? (int)gridDim.x / (a.nchan / kCh) : kRenormSplit;
+    const int part = blockIdx.x % nparts, c0 = (blockIdx.x / nparts) * kCh, c = c0 + 4 * q;
+    const int st = blockIdx.y % a.nstokes, p = blockIdx.y / a.nstokes, cc = blockIdx.z;
+    const long long sstride = (long long)a.nstokes * a.nchan;
+    const float *S = a.S + cc * a.S_cc + ((long long)p * a.nstep * a.nstokes + st) * a.nchan + c;
+    const int sb = (int)((long long)a.nstep * part / nparts), se = (int)((long long)a.nstep * (part + 1) / nparts);
+    const long long si = cc * a.stat_cc + ((long long)p * a.nstokes + st) * a.nchan + c0;
+
+    float lo = 0.f, hi = 0.f; // thread t < kCh: the extremes of channel c0 + t
+    if (kStats) {
+        if (tid < kCh) {
+            const bool nan0 = a.st_nan0[si + tid] != 0;
+            lo = nan0 ? __int_as_float(0x7fffffff) : fkey_inv(a.st_mn[si + tid]);
+            hi = nan0 ? __int_as_float(0x7fffffff) : fkey_inv(a.st_mx[si + tid]);
+        }
+    } else {
+        cg::cluster_group cluster = cg::this_cluster();
+        for (int s = sb + row; s < se; s += kRows)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&rsm[(s - sb) * kQ + q])),
+                         "l"(S + s * sstride)
+                         : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        float4 mn = *reinterpret_cast<const float4 *>(S), mx = mn;
+        asm volatile("cp.async.wait_group 0;" ::: "memory"); // each thread scans what it copied
+        for (int s = sb + row; s < se; s += kRows) {
+            const float4 v = rsm[(s - sb) * kQ + q];
+            mn = min4(mn, v);
+            mx = max4(mx, v);
+        }
+        // the warp's rows, then the block's warps, then the cluster's blocks
+#pragma unroll
+        for (int o = kQ; o < 32; o <<= 1) {
+            mn = min4(mn, shfl4(mn, o));
+            mx = max4(mx, shfl4(mx, o));
+        }
+        if ((tid & 31) < kQ) {
+            smin[tid >> 5][q] = mn;
+            smax[tid >> 5][q] = mx;
+        }
+        __syncthreads();
+        float *bmin = &smin[0][0].x, *bmax = &smax[0][0].x;
+        if (tid < kCh)
+            for (int w = 1; w < kThr / 32; w++) {
+                bmin[tid] = fminf(bmin[tid], bmin[w * kCh + tid]);
+                bmax[tid] = fmaxf(bmax[tid], bmax[w * kCh + tid]);
+            }
+        cluster.sync(); // every block's partials are in its shared memory
+        if (tid < kCh) {
+            // a NaN first value makes both extremes NaN, other NaN are skipped
+            const float s0 = a.S[(S - a.S) - 4 * q + tid];
+            lo = hi = s0;
+#pragma unroll
+            for (int r = 0; r < kRenormSplit; r++) {
+                lo = fminf(lo, cluster.map_shared_rank(bmin, r)[tid]);
+                hi = fmaxf(hi, cluster.map_shared_rank(bmax, r)[tid]);
+            }
+            if (isnan(s0)) lo = hi = s0;
+        }
+        // no block leaves while another still reads its partials: arrive now
+        // (the reads are done, nothing is published), wait at the end
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    }
+    if (tid < kCh) {
+        const float scale = (float)((double)(hi - lo) / 256.0);
+        s_par[0][tid] = lo;
+        s_par[1][tid] = scale;
+        s_par[2][tid] = 1.f / scale;
+        if (part == 0) {
+            a.scales[si + tid] = scale;
+            a.offsets[si + tid] = lo;
+        }
+    }
+    __syncthreads();
+    const float4 off = *reinterpret_cast<const float4 *>(&s_par[0][4 * q]);
+    const float4 scl = *reinterpret_cast<const float4 *>(&s_par[1][4 * q]);
+    const float4 rcp = *reinterpret_cast<const float4 *>(&s_par[2][4 * q]);
+    uint8_t *o = a.out + cc * a.out_cc + p * a.out_p + st * a.out_st + c;
+    auto put = [&](int s, float4 v) { *reinterpret_cast<uint32_t *>(o + (long long)s * a.out_s) = quant4_u8(v, off, scl, rcp); };
+    if (kStats) {
+        int s = sb + row;
+        for (; s + 3 * kRows < se; s += 4 * kRows) { // four loads in flight
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = __ldcs(reinterpret_cast<const float4 *>(S + (s + u * kRows) * sstride));
+#pragma unroll
+            for (int u = 0; u < 4; u++) put(s + u * kRows, v[u]);
+        }
+        for (; s < se; s += kRows) put(s, *reinterpret_cast<const float4 *>(S + s * sstride));
+    } else {
+#pragma unroll 2
+        for (int s = sb + row; s < se; s += kRows) put(s, rsm[(s - sb) * kQ + q]);
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    }
+}
+
+template <int kCh, bool kStats> static int launch_renorm4(const RenormArgs &a, int ncc, cudaStream_t st)
+{
+    auto kern = renorm4_kernel<kCh, kStats>;
+    cudaLaunchConfig_t cfg = {};
+    // with the extremes given: enough blocks for four per SM
+    const long long groups = (long long)(a.nchan / kCh) * a.npointing * a.nstokes * ncc;
+    const long long parts = kStats ? std::max(1LL, std::min<long long>(a.nstep / 256 + 1, (8 * 152 + groups - 1) / groups))
+                                   : kRenormSplit;
+    cfg.gridDim = dim3((unsigned)(parts * (a.nchan / kCh)), a.npointing * a.nstokes, ncc);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kStats ? 1 : kRenormSplit;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (!kStats) {
+        cfg.dynamicSmemBytes = sizeof(float) * kCh * (size_t)((a.nstep + kRenormSplit - 1) / kRenormSplit);
+        const int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRenormTile),
+                                  "cudaFuncSetAttribute(renorm4)");
+        if (rc) return rc;
+    }
+    const int rc = check_cuda(cudaLaunchKernelEx(&cfg, kern, a), "cudaLaunchKernelEx(renorm4_kernel)");
+    return rc ? rc : check_launch("renorm4_kernel");
+}
+
 int launch_renorm(const RenormArgs &a, int ncc, cudaStream_t st)
 {
     if (a.nstep <= 0 || ncc <= 0) return VGB_SUCCESS;
+    const auto low = [](const void *p) { return reinterpret_cast<uintptr_t>(p) & 15; };
+    const bool aligned = !low(a.S) && !low(a.scales) && !low(a.offsets) && a.nchan % 32 == 0 && (low(a.out) & 3) == 0 &&
+                         ((a.out_cc | a.out_p | a.out_s | a.out_st) & 3) == 0 && a.S_cc % 4 == 0 && a.stat_cc % 4 == 0;
+    if (aligned && a.st_mn) return launch_renorm4<32, true>(a, ncc, st);
+    const long long share = (long long)((a.nstep + kRenormSplit - 1) / kRenormSplit) * 4; // bytes per channel
+    if (aligned && share * 32 <= kRenormTile) return launch_renorm4<32, false>(a, ncc, st);
+    if (aligned && share * 16 <= kRenormTile) return launch_renorm4<16, false>(a, ncc, st);
+    if (aligned && share * 8 <= kRenormTile) return launch_renorm4<8, false>(a, ncc, st);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(kRenormSplit * ((a.nchan + 31) / 32), a.npointing * a.nstokes, ncc);
     cfg.blockDim = dim3(256);

@@ -174,6 +174,33 @@ __device__ __forceinline__ uint8_t quant_u8(float e, float off, float scl, float
     return sat_u8_half(x / scl);
 }
 
+// quant_u8 of four values as one word (byte k = value k). One test covers the
+// four: with the offset at most every value, q0 is never below zero and the
+// byte is the low byte of q0 + 1.5 * 2^23 wherever quant_u8 takes its short
+// way (8 instead of 20 instructions per value); otherwise quant_u8 itself.
+static __device__ __noinline__ uint32_t quant4_slow(float4 e, float4 off, float4 scl, float4 rcp)
+{
+    return (uint32_t)quant_u8(e.x, off.x, scl.x, rcp.x) | ((uint32_t)quant_u8(e.y, off.y, scl.y, rcp.y) << 8) |
+           ((uint32_t)quant_u8(e.z, off.z, scl.z, rcp.z) << 16) | ((uint32_t)quant_u8(e.w, off.w, scl.w, rcp.w) << 24);
+}
+
+__device__ __forceinline__ bool quant_short(float e, float off, float rcp, uint32_t &bits)
+{
+    const float q0 = __fmul_rn(__fsub_rn(e, off), rcp);
+    const float y = __fadd_rn(q0, 12582912.f);
+    bits = __float_as_uint(y);
+    return q0 >= 0.f && q0 < 512.f && fabsf(__fsub_rn(q0, __fsub_rn(y, 12582912.f))) < 0.499755859375f;
+}
+
+__device__ __forceinline__ uint32_t quant4_u8(float4 e, float4 off, float4 scl, float4 rcp)
+{
+    uint32_t b[4];
+    const bool s0 = quant_short(e.x, off.x, rcp.x, b[0]), s1 = quant_short(e.y, off.y, rcp.y, b[1]);
+    const bool s2 = quant_short(e.z, off.z, rcp.z, b[2]), s3 = quant_short(e.w, off.w, rcp.w, b[3]);
+    if (!(s0 && s1 && s2 && s3)) return quant4_slow(e, off, scl, rcp);
+    return __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+}
+
 // 1-D bulk copy global -> shared through the TMA unit. dst, src and bytes
 // must be multiples of 16 (callers copy whole 256-byte frames).
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
@@ -318,6 +345,31 @@ constexpr int kFftRow = 152;
 // of 128 float2: pairs k1 = 2i, 2i + 1 of one j sit together, so pass 1 reads
 // two twiddles per 16-byte load.
 __host__ __device__ __forceinline__ int fft128_tw_slot(int k1, int j) { return ((k1 >> 1) * 8 + j) * 2 + (k1 & 1); }
+
+// cos(pi m / 64), m = 0 .. 127, each the FP32 value nearest to the FP64 one. A
+// table instead of FP64 sine and cosine in every CTA, whose latency showed at
+// the start of short kernels.
+static __device__ const float kCos128[128] = {
+    1.0f, 0.99879545f, 0.99518472f, 0.989176512f, 0.980785251f, 0.970031261f, 0.956940353f, 0.941544056f,
+    0.923879504f, 0.903989315f, 0.881921291f, 0.857728601f, 0.831469595f, 0.803207517f, 0.773010433f, 0.740951121f,
+    0.707106769f, 0.671558976f, 0.634393275f, 0.59569931f, 0.555570245f, 0.514102757f, 0.471396744f, 0.427555084f,
+    0.382683426f, 0.336889863f, 0.290284663f, 0.242980182f, 0.195090324f, 0.146730468f, 0.0980171412f, 0.0490676761f,
+    0.0f, -0.0490676761f, -0.0980171412f, -0.146730468f, -0.195090324f, -0.242980182f, -0.290284663f, -0.336889863f,
+    -0.382683426f, -0.427555084f, -0.471396744f, -0.514102757f, -0.555570245f, -0.59569931f, -0.634393275f, -0.671558976f,
+    -0.707106769f, -0.740951121f, -0.773010433f, -0.803207517f, -0.831469595f, -0.857728601f, -0.881921291f, -0.903989315f,
+    -0.923879504f, -0.941544056f, -0.956940353f, -0.970031261f, -0.980785251f, -0.989176512f, -0.99518472f, -0.99879545f,
+    -1.0f, -0.99879545f, -0.99518472f, -0.989176512f, -0.980785251f, -0.970031261f, -0.956940353f, -0.941544056f,
+    -0.923879504f, -0.903989315f, -0.881921291f, -0.857728601f, -0.831469595f, -0.803207517f, -0.773010433f, -0.740951121f,
+    -0.707106769f, -0.671558976f, -0.634393275f, -0.59569931f, -0.555570245f, -0.514102757f, -0.471396744f, -0.427555084f,
+    -0.382683426f, -0.336889863f, -0.290284663f, -0.242980182f, -0.195090324f, -0.146730468f, -0.0980171412f, -0.0490676761f,
+    0.0f, 0.0490676761f, 0.0980171412f, 0.146730468f, 0.195090324f, 0.242980182f, 0.290284663f, 0.336889863f,
+    0.382683426f, 0.427555084f, 0.471396744f, 0.514102757f, 0.555570245f, 0.59569931f, 0.634393275f, 0.671558976f,
+    0.707106769f, 0.740951121f, 0.773010433f, 0.803207517f, 0.831469595f, 0.857728601f, 0.881921291f, 0.903989315f,
+    0.923879504f, 0.941544056f, 0.956940353f, 0.970031261f, 0.980785251f, 0.989176512f, 0.99518472f, 0.99879545f,
+};
+
+// W128^m = (cos, sin) of 2 pi m / 128, m >= 0.
+__device__ __forceinline__ float2 w128(int m) { return make_float2(__ldg(&kCos128[m & 127]), __ldg(&kCos128[(m + 96) & 127])); }
 
 // Pass 1: the 8 threads of one group read x[8q + j] (row `row`), transform
 // over q, twiddle by W128^{j k1} from `tw` (cos/sin pairs of the positive
