@@ -35,11 +35,15 @@ __device__ __forceinline__ uint32_t vdif_advanced_word(uint32_t w0, uint32_t w1,
     return (w1 & 0xFF000000u) | (total - sec * (uint32_t)kVdifFramesPerSecond);
 }
 
-constexpr int kIFT = 32;                 // frames per CTA
-constexpr int kIThreads = 512;           // two halves of 256: 16 frames each in the polyphase sum
+// Frames per CTA: a second's 10,000 are 304 CTAs of 33, two for each of the 152
+// SMs (32 frames made 313 of them, and a second wave for the last nine: one
+// channel's second 20.8 -> 15.4 us).
+constexpr int kIFT = 33;
+constexpr int kIThreads = 512;           // two halves of 256: 17 and 16 frames in the polyphase sum
+constexpr int kIHalf = (kIFT + 1) / 2;
 
-constexpr int kIRowsPad = 88;            // 2 x (kIFT + 11) = 86 rows, padded to whole warps of
-                                         // 8-thread groups; ~108 KB: two CTAs per SM
+constexpr int kIRowsPad = 88;            // 2 x (kIFT + 11) rows, whole warps of 8-thread groups;
+                                         // ~108 KB: two CTAs per SM
 static_assert(kIRowsPad >= 2 * (kIFT + kP - 1) && kIRowsPad % 4 == 0, "FFT rows");
 
 
@@ -60,9 +64,7 @@ __global__ void __launch_bounds__(kIThreads, 2) ipfb_kernel(const IpfbArgs a)
 
     if (tid < 128) {
         const int k1 = tid >> 3, j = tid & 7;
-        double sn, cs;
-        sincospi((double)(j * k1) / 64.0, &sn, &cs);
-        sm.tw[fft128_tw_slot(k1, j)] = make_float2((float)cs, (float)sn);
+        sm.tw[fft128_tw_slot(k1, j)] = w128(j * k1);
     }
     // load X_k[m] for m in [f0 - 11, f0 + kIFT), de-interleaving the pols
     const float4 *e = a.e + job * a.e_job;
@@ -116,7 +118,7 @@ __global__ void __launch_bounds__(kIThreads, 2) ipfb_kernel(const IpfbArgs a)
     }
     __syncthreads();
 
-    // polyphase sum: thread (r, pol) of half h sums frames 16 h .. 16 h + 15
+    // polyphase sum: thread (r, pol) of half h sums frames kIHalf h ..
     const int r = (tid & 255) >> 1, pol = tid & 1, half = tid >> 8;
     float fr[kP];
 #pragma unroll
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(kIThreads, 2) ipfb_kernel(const IpfbArgs a)
     const float invK = 1.0f / kK;
     float *outf = a.out_f ? a.out_f + job * a.outf_job : nullptr;
     uint8_t *vd = a.vdif ? a.vdif + job * a.vdif_job : nullptr;
-    // frame headers: one word per thread (kIFT frames x 8 words = 256)
+    // frame headers: one word per thread (kIFT frames x 8 words)
     if (vd && tid < kIFT * 8) {
         const int f = f0 + (tid >> 3), wi = tid & 7;
         if (f < a.nsamples) {
@@ -137,29 +139,31 @@ __global__ void __launch_bounds__(kIThreads, 2) ipfb_kernel(const IpfbArgs a)
             reinterpret_cast<uint32_t *>(vd + (long long)f * 544)[wi] = wv;
         }
     }
-    static_assert(kIThreads == 512 && kIFT == 32, "two halves of 16 frames");
+    static_assert(kIThreads == 512 && kIFT * 8 <= kIThreads, "two halves; a header word per thread");
     {
-        const int chunk = 16 * half;
-        float ar[16], ai[16];
+        const int chunk = kIHalf * half;
+        float ar[kIHalf], ai[kIHalf];
 #pragma unroll
-        for (int q = 0; q < 16; q++) ar[q] = ai[q] = 0.f;
-        // frame fl = chunk + q uses local m index (chunk + q) + 11 - p
+        for (int q = 0; q < kIHalf; q++) ar[q] = ai[q] = 0.f;
+        // frame fl = chunk + q uses local m index (chunk + q) + 11 - p; the
+        // second half's last window row is past the rows when kIFT is odd
 #pragma unroll
-        for (int w = 0; w < 16 + kP - 1; w++) {
+        for (int w = 0; w < kIHalf + kP - 1; w++) {
+            if (w == kIHalf + kP - 2 && 2 * kIHalf > kIFT && half) break;
             const float2 y = sm.y[2 * (chunk + w) + pol][r];
 #pragma unroll
             for (int p = 0; p < kP; p++) {
                 const int q = w - (kP - 1) + p;
-                if (q >= 0 && q < 16) {
+                if (q >= 0 && q < kIHalf) {
                     ar[q] = fmaf(fr[p], y.x, ar[q]);
                     ai[q] = fmaf(fr[p], y.y, ai[q]);
                 }
             }
         }
 #pragma unroll
-        for (int q = 0; q < 16; q++) {
+        for (int q = 0; q < kIHalf; q++) {
             const int f = f0 + chunk + q;
-            if (f >= a.nsamples) break;
+            if (f >= a.nsamples || chunk + q >= kIFT) break;
             const float xr = ar[q] * invK, xi = ai[q] * invK;
             const long long n = (long long)f * kK + r;
             if (outf) reinterpret_cast<float2 *>(outf)[n * 2 + pol] = make_float2(xr, xi);
@@ -273,9 +277,7 @@ __global__ void __launch_bounds__(256) fft_staged_kernel(float2 *rows, long long
     const long long r0 = blockIdx.x * 32LL;
     if (tid < 128) {
         const int k1 = tid >> 3, j = tid & 7;
-        double sn, cs;
-        sincospi((double)(j * k1) / 64.0, &sn, &cs);
-        tw[fft128_tw_slot(k1, j)] = make_float2((float)cs, (float)sn);
+        tw[fft128_tw_slot(k1, j)] = w128(j * k1);
     }
     for (int idx = tid; idx < 32 * kK; idx += 256) {
         const int r = idx / kK, n = idx % kK;

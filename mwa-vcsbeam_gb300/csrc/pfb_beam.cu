@@ -380,9 +380,7 @@ __device__ __forceinline__ void init_twiddles(float2 *tw, int tid)
 {
     if (tid < 128) {
         const int k1 = tid >> 3, j = tid & 7;
-        double sn, cs;
-        sincospi((double)(j * k1) / 64.0, &sn, &cs);
-        tw[fft128_tw_slot(k1, j)] = make_float2((float)cs, (float)sn);
+        tw[fft128_tw_slot(k1, j)] = w128(j * k1);
     }
 }
 
