@@ -331,11 +331,18 @@ __device__ __forceinline__ void wola_step(FrontSmemT<G> &sm, int s, int li, int 
     wola_rows<kW, kFpga>(sm.stage[s][li][0], &sm.buf[li * kT], n0, t);
 }
 
-// vcsbeam.h.in:453-456: (int)round(x) clipped to [-8, 7].
-__device__ __forceinline__ float demote4(float x)
+// vcsbeam.h.in:453-456: (int)round(x) clipped to [-8, 7], x = X * scale (a
+// power of two). Clipped first (the bounds are whole numbers), then half away
+// from zero as the truncation of |x| + 1/2 rounded towards zero, which never
+// reaches the next whole number from below: 5 instructions where roundf, the
+// scaling and the clipping took 11 (of 358 per input spectrum's 8 values a
+// thread, with the --smart mode bound by issue).
+template <bool kScale> __device__ __forceinline__ float demote4(float X)
 {
-    float r = roundf(x);
-    return fminf(fmaxf(r, -8.0f), 7.0f);
+    constexpr float kBound = kScale ? (float)kK : 1.0f;
+    const float y = fminf(fmaxf(X, -8.0f * kBound), 7.0f * kBound);
+    const float half = copysignf(0.5f, y);
+    return truncf(kScale ? __fmaf_rz(y, 1.0f / kK, half) : __fadd_rz(y, half));
 }
 
 // Steps 4-5: FFT of row g = (li, m) by the 8 threads of a group, in place;
@@ -360,12 +367,8 @@ __device__ __forceinline__ void fft_rows(float2 (*buf)[kFftRow], const float2 *t
             const int k = fft128_index(j, h, k2);
             const int kp = (k + kK / 2) & (kK - 1);
             const float2 X = out[h][k2];
-            float vr = kScale ? X.y * (1.0f / kK) : X.y, vi = kScale ? X.x * (1.0f / kK) : X.x;
-            if (kDemote) {
-                vr = demote4(vr);
-                vi = demote4(vi);
-            }
-            row[kp] = make_float2(vr, vi);
+            if (kDemote) row[kp] = make_float2(demote4<kScale>(X.y), demote4<kScale>(X.x));
+            else row[kp] = kScale ? make_float2(X.y * (1.0f / kK), X.x * (1.0f / kK)) : make_float2(X.y, X.x);
         }
 }
 
