@@ -96,14 +96,14 @@ __device__ __forceinline__ uint32_t issue_frames(const VoltView &vv, int cc, int
 // may be consumed before it is posted; the phase still cannot complete before
 // warp 0's arrival. Called by every thread after the step's first block
 // barrier.
-template <int G>
+template <int G, int T = kT>
 __device__ __forceinline__ void produce_spread(FrontSmemT<G> &sm, const VoltView &vv, int cc, int it, int m0,
                                               int nspectra, const CUtensorMap *wmap, unsigned *status)
 {
     if ((threadIdx.x & 31) != 0) return;
     const int warp = threadIdx.x >> 5;
     const int s = it & 1;
-    const int w_end = min(m0 + kWin, nspectra + kP - 1);
+    const int w_end = min(m0 + T + kP - 1, nspectra + kP - 1);
     const uint32_t per_input = (w_end - m0) * kFrameBytes;
     constexpr uint32_t kWBytes = (G / 2) * kK * 16;   // one Jones row of G/2 tiles
     if (warp == 0) {
@@ -216,25 +216,25 @@ __device__ __forceinline__ void make_taps(const int (&hc)[2][kP], typename WolaT
     }
 }
 
-// stage_in: the input's kWin staged frames [w][kK]; rows: its kT output rows.
-template <int kW, bool kFpga>
+// stage_in: the input's staged frames [w][kK]; rows: its T output rows.
+template <int kW, bool kFpga, int T = kT>
 __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[kFftRow], int n0,
                                           const typename WolaTap<kW>::type (&t)[kP])
 {
     static_assert(kW != kWolaSplit || !kFpga, "the split sum is for the unrounded mode");
     const uint32_t *x = reinterpret_cast<const uint32_t *>(stage_in + n0);
     if constexpr (kW == kWolaInt32) {
-        int ar[kT][2], ai[kT][2];
+        int ar[T][2], ai[T][2];
 #pragma unroll
-        for (int m = 0; m < kT; m++) ar[m][0] = ar[m][1] = ai[m][0] = ai[m][1] = 0;
+        for (int m = 0; m < T; m++) ar[m][0] = ar[m][1] = ai[m][0] = ai[m][1] = 0;
 #pragma unroll
-        for (int w = 0; w < kWin; w++) {
+        for (int w = 0; w < T + kP - 1; w++) {
             int xr[2], xi[2];
             c4_to_i(x[w * (kK / 2)], xr, xi);
 #pragma unroll
             for (int p = 0; p < kP; p++) {
                 const int m = w - p;
-                if (m >= 0 && m < kT) {
+                if (m >= 0 && m < T) {
 #pragma unroll
                     for (int q = 0; q < 2; q++) {
                         const int h = q ? t[p].y : t[p].x;
@@ -245,7 +245,7 @@ __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[
             }
         }
 #pragma unroll
-        for (int m = 0; m < kT; m++) {
+        for (int m = 0; m < T; m++) {
             float4 b;
             if (kFpga) {
                 int v[4] = {ar[m][0], ai[m][0], ar[m][1], ai[m][1]};
@@ -260,13 +260,12 @@ __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[
             *reinterpret_cast<float4 *>(&rows[m][n0]) = b;
         }
     } else if constexpr (kW == kWolaSplit) {
-        // Two passes of kT / 2 spectra each keep the even and odd sums within
-        // the FP32 path's registers; each pass reads the kT / 2 + kP - 1
+        // Passes of at most kT / 2 spectra each keep the even and odd sums within
+        // the FP32 path's registers; each pass reads the kH + kP - 1
         // frames its spectra need.
-        constexpr int kH = kT / 2;
+        constexpr int kH = T < kT / 2 ? T : kT / 2;
 #pragma unroll
-        for (int half = 0; half < 2; half++) {
-            const int mb = half * kH;
+        for (int mb = 0; mb < T; mb += kH) {
             float2 er[kH], ei[kH], od_r[kH], od_i[kH];
 #pragma unroll
             for (int m = 0; m < kH; m++) er[m] = ei[m] = od_r[m] = od_i[m] = make_float2(0.f, 0.f);
@@ -295,24 +294,24 @@ __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[
             }
         }
     } else {
-        float2 ar[kT], ai[kT];
+        float2 ar[T], ai[T];
 #pragma unroll
-        for (int m = 0; m < kT; m++) ar[m] = ai[m] = make_float2(0.f, 0.f);
+        for (int m = 0; m < T; m++) ar[m] = ai[m] = make_float2(0.f, 0.f);
 #pragma unroll
-        for (int w = 0; w < kWin; w++) {
+        for (int w = 0; w < T + kP - 1; w++) {
             float2 xr, xi;
             widen4<kFpga>(x[w * (kK / 2)], xr, xi);
 #pragma unroll
             for (int p = 0; p < kP; p++) {
                 const int m = w - p;
-                if (m >= 0 && m < kT) {
+                if (m >= 0 && m < T) {
                     ar[m] = __ffma2_rn(t[p], xr, ar[m]);
                     ai[m] = __ffma2_rn(t[p], xi, ai[m]);
                 }
             }
         }
 #pragma unroll
-        for (int m = 0; m < kT; m++) {
+        for (int m = 0; m < T; m++) {
             float4 b;
             if (kFpga) {
                 b = make_float4(fpga_round(ar[m].x), fpga_round(ai[m].x), fpga_round(ar[m].y), fpga_round(ai[m].y));
@@ -324,11 +323,11 @@ __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[
     }
 }
 
-template <int kW, bool kFpga, int G>
+template <int kW, bool kFpga, int G, int T = kT>
 __device__ __forceinline__ void wola_step(FrontSmemT<G> &sm, int s, int li, int n0,
                                           const typename WolaTap<kW>::type (&t)[kP])
 {
-    wola_rows<kW, kFpga>(sm.stage[s][li][0], &sm.buf[li * kT], n0, t);
+    wola_rows<kW, kFpga, T>(sm.stage[s][li][0], &sm.buf[li * kT], n0, t);
 }
 
 // vcsbeam.h.in:453-456: (int)round(x) clipped to [-8, 7], x = X * scale (a
@@ -515,21 +514,19 @@ __device__ __forceinline__ void beam_store_extremes(const BeamArgs &a, int cc, i
 // G = 8 (one CTA of 512 threads, half the steps and block barriers per
 // input). Every (k', m) is summed by one thread over the tiles in the same
 // order either way, so both give identical results; the host picks by timing.
-template <int kW, bool kFpga, bool kDemote, int G>
-__global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
-    beam_kernel(const BeamArgs a, const __grid_constant__ CUtensorMap wmap)
+// T: spectra of this CTA (kT, or fewer where the last wave of CTAs would be
+// nearly empty); row m of an input is row li * kT + m whatever T.
+template <int kW, bool kFpga, bool kDemote, int G, int T>
+__device__ __forceinline__ void beam_body(const BeamArgs &a, const CUtensorMap *wmap, FrontSmemT<G> &sm, int cc, int m0)
 {
     constexpr int kTiles = G / 2;        // tiles per step
     constexpr int kMh = G / 2;           // threads per k' (spectra m = mh + kMh mi)
-    constexpr int kMi = kT / kMh;        // spectra per thread
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    FrontSmemT<G> &sm = *reinterpret_cast<FrontSmemT<G> *>(smem_raw);
+    constexpr int kMi = T / kMh;         // spectra per thread
+    static_assert(T % kMh == 0 && T <= kT, "whole spectra per thread");
     const int tid = threadIdx.x;
-    const int cc = blockIdx.y;
-    const int m0 = blockIdx.x * kT;
     const int nsteps = (a.vv.ninputs + G - 1) / G;
 
-    if (tid == 0) prefetch_tmap(&wmap);
+    if (tid == 0) prefetch_tmap(wmap);
     init_front(sm, tid);
     typename WolaTap<kW>::type tp[kP];
     const int li = tid >> 6, n0 = 2 * (tid & 63);
@@ -539,7 +536,7 @@ __global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
         make_taps<kW, kFpga>(hc, tp);
     }
     __syncthreads();
-    produce_spread(sm, a.vv, cc, 0, m0, a.nspectra, &wmap, a.status);
+    produce_spread<G, T>(sm, a.vv, cc, 0, m0, a.nspectra, wmap, a.status);
 
     // beam accumulators for (k', m = mh + kMh mi)
     const int kp = tid & (kK - 1), mh = tid >> 7;
@@ -555,10 +552,12 @@ __global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
             return;
         }
         // everyone has finished step it-1, so its buffers may be refilled
-        if (it + 1 < nsteps) produce_spread(sm, a.vv, cc, it + 1, m0, a.nspectra, &wmap, a.status);
-        wola_step<kW, kFpga>(sm, it & 1, li, n0, tp);
+        if (it + 1 < nsteps) produce_spread<G, T>(sm, a.vv, cc, it + 1, m0, a.nspectra, wmap, a.status);
+        wola_step<kW, kFpga, G, T>(sm, it & 1, li, n0, tp);
         input_barrier(li);
-        fft_step<kDemote, kFpga>(sm, tid);
+        // a warp transforms rows 4 (warp % 2) .. + 3 of its input (rows past
+        // the T-th hold leftovers nobody reads)
+        if (T == kT || ((tid >> 5) & 1) * 4 < T) fft_step<kDemote, kFpga>(sm, tid);
         __syncthreads();
 #pragma unroll
         for (int aa = 0; aa < kTiles; aa++) {
@@ -578,6 +577,22 @@ __global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
 #pragma unroll
     for (int mi = 0; mi < kMi; mi++) beam_store(a, cc, m0 + mh + kMh * mi, kp, acc[mi], kmn, kmx);
     beam_store_extremes(a, cc, kp, kmn, kmx);
+}
+
+// CTAs 0 .. ncc n8 - 1: the first n8 tiles of kT spectra of every channel; the
+// rest: ntail tiles of kTail spectra each.
+template <int kW, bool kFpga, bool kDemote, int G, int kTail>
+__global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
+    beam_kernel(const BeamArgs a, const __grid_constant__ CUtensorMap wmap)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    FrontSmemT<G> &sm = *reinterpret_cast<FrontSmemT<G> *>(smem_raw);
+    const int b = blockIdx.x, n = a.ncc * a.n8;
+    if (b < n) {
+        beam_body<kW, kFpga, kDemote, G, kT>(a, &wmap, sm, b / a.n8, b % a.n8 * kT);
+    } else if constexpr (kTail < kT) {
+        beam_body<kW, kFpga, kDemote, G, kTail>(a, &wmap, sm, (b - n) / a.ntail, a.n8 * kT + (b - n) % a.ntail * kTail);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1243,6 +1258,41 @@ static int dispatch(const Args &a, dim3 grid, int wola, bool fpga, bool demote, 
 static std::atomic<int> g_pfb_variant{0}; // 0: autotuned; else the forced variant (3, 4, 5 or 8)
 static std::atomic<int> g_pfb_last{0};    // inputs per step of the last fused launch
 
+// Tiles of beam_kernel with `per_sm` CTAs per SM: whole waves of kT spectra per
+// CTA, and the spectra left over in tiles of 2 (`least` 2) or 4 where that fills
+// at most one more wave. A second of one channel is 1,250 tiles of 8 on 304
+// places, 34 of them in a fifth wave: 4 x 304 tiles and 136 of 2 spectra take
+// 0.94 instead of 0.99 ms. A CTA of 2 spectra converts 13 frames for them and
+// takes about a third of a full one's time, so nothing else is split. Returns
+// the spectra of a leftover tile.
+static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least)
+{
+    static std::atomic<int> sms{0};
+    if (!sms.load()) {
+        int dev = 0, n = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+            n <= 0) {
+            cudaGetLastError();
+            n = 152;
+        }
+        sms = n;
+    }
+    const long long slots = (long long)per_sm * sms.load(), total = (long long)a.nspectra * ncc;
+    a.ncc = ncc;
+    const long long full = total / (kT * slots) * slots; // tiles in whole waves
+    const int n8 = (int)std::min<long long>(full / ncc, a.nspectra / kT);
+    const int left = a.nspectra - n8 * kT;
+    for (int t = least; t < kT; t *= 2)
+        if (left > 0 && (long long)((left + t - 1) / t) * ncc <= slots) {
+            a.n8 = n8;
+            a.ntail = (left + t - 1) / t;
+            return t;
+        }
+    a.n8 = (a.nspectra + kT - 1) / kT;
+    a.ntail = 0;
+    return 4;
+}
+
 template <int A, bool B, bool C> struct BeamSel {
     static int run_g(const BeamArgs &a, dim3 grid, cudaStream_t st, int g)
     {
@@ -1269,11 +1319,16 @@ template <int A, bool B, bool C> struct BeamSel {
                 return rc;
             kern<<<grid, kWsThreads, sizeof(WsSmem), st>>>(a, wmap);
         } else if (g == 8) {
-            if ((rc = prep<8>(beam_kernel<A, B, C, 8>))) return rc;
-            beam_kernel<A, B, C, 8><<<grid, 512, front_smem<8>(), st>>>(a, wmap);
+            BeamArgs b = a;
+            beam_tiles(b, (int)grid.y, 1, 4);
+            if ((rc = prep<8>(beam_kernel<A, B, C, 8, 4>))) return rc;
+            beam_kernel<A, B, C, 8, 4><<<b.ncc * (b.n8 + b.ntail), 512, front_smem<8>(), st>>>(b, wmap);
         } else {
-            if ((rc = prep<4>(beam_kernel<A, B, C, 4>))) return rc;
-            beam_kernel<A, B, C, 4><<<grid, 256, front_smem<4>(), st>>>(a, wmap);
+            BeamArgs b = a;
+            const int tail = beam_tiles(b, (int)grid.y, 2, 2);
+            auto kern = tail == 2 ? beam_kernel<A, B, C, 4, 2> : beam_kernel<A, B, C, 4, 4>;
+            if ((rc = prep<4>(kern))) return rc;
+            kern<<<b.ncc * (b.n8 + b.ntail), 256, front_smem<4>(), st>>>(b, wmap);
         }
         return check_launch("beam_kernel");
     }

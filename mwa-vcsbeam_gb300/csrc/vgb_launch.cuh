@@ -30,6 +30,8 @@ struct BeamArgs {
     // only make sure the kernel variant of this shape is chosen (launches
     // nothing where it is known already)
     bool choose_only;
+    // set by the launcher: channels, and tiles of 8 and of fewer spectra per channel
+    int ncc, n8, ntail;
 };
 
 struct PackArgs {
