@@ -217,7 +217,7 @@ __device__ __forceinline__ void make_taps(const int (&hc)[2][kP], typename WolaT
 }
 
 // stage_in: the input's staged frames [w][kK]; rows: its T output rows.
-template <int kW, bool kFpga, int T = kT>
+template <int kW, bool kFpga, int T = kT, int kPassMax = kT / 2>
 __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[kFftRow], int n0,
                                           const typename WolaTap<kW>::type (&t)[kP])
 {
@@ -260,10 +260,10 @@ __device__ __forceinline__ void wola_rows(const char2 *stage_in, float2 (*rows)[
             *reinterpret_cast<float4 *>(&rows[m][n0]) = b;
         }
     } else if constexpr (kW == kWolaSplit) {
-        // Passes of at most kT / 2 spectra each keep the even and odd sums within
+        // Passes of at most kPassMax spectra each keep the even and odd sums within
         // the FP32 path's registers; each pass reads the kH + kP - 1
         // frames its spectra need.
-        constexpr int kH = T < kT / 2 ? T : kT / 2;
+        constexpr int kH = T < kPassMax ? T : kPassMax;
 #pragma unroll
         for (int mb = 0; mb < T; mb += kH) {
             float2 er[kH], ei[kH], od_r[kH], od_i[kH];
@@ -349,12 +349,12 @@ template <bool kScale> __device__ __forceinline__ float demote4(float X)
 // kScale: apply the 1/K here (after FPGA rounding); without FPGA rounding the
 // WOLA output already carries it (scaling by a power of two commutes exactly
 // with the FFT's arithmetic).
-template <bool kDemote, bool kScale>
-__device__ __forceinline__ void fft_rows(float2 (*buf)[kFftRow], const float2 *tw, int tid)
+template <bool kDemote, bool kScale, class Pass1>
+__device__ __forceinline__ void fft_rows_with(float2 (*buf)[kFftRow], int tid, Pass1 &&pass1)
 {
     const int g = tid >> 3, j = tid & 7;
     float2 *row = buf[g];
-    fft128_pass1<-1>(row, tw, j);
+    pass1(row, j);
     __syncwarp();
     float2 out[2][8];
     fft128_pass2<-1>(row, j, out);
@@ -369,6 +369,86 @@ __device__ __forceinline__ void fft_rows(float2 (*buf)[kFftRow], const float2 *t
             if (kDemote) row[kp] = make_float2(demote4<kScale>(X.y), demote4<kScale>(X.x));
             else row[kp] = kScale ? make_float2(X.y * (1.0f / kK), X.x * (1.0f / kK)) : make_float2(X.y, X.x);
         }
+}
+
+template <bool kDemote, bool kScale>
+__device__ __forceinline__ void fft_rows(float2 (*buf)[kFftRow], const float2 *tw, int tid)
+{
+    fft_rows_with<kDemote, kScale>(buf, tid, [&](float2 *row, int j) { fft128_pass1<-1>(row, tw, j); });
+}
+
+// Taps of samples n0, n0+1: h[K P - K p - n - 1] (pfb.cpp:159).
+__device__ __forceinline__ void load_taps(const int *filter, int n0, int (&hc)[2][kP])
+{
+#pragma unroll
+    for (int q = 0; q < 2; q++)
+#pragma unroll
+        for (int p = 0; p < kP; p++) hc[q][p] = __ldg(filter + kK * kP - kK * p - (n0 + q) - 1);
+}
+
+// A thread's taps (24 words) and twiddles (W128^{j k1}, j = tid % 8, k1 = 1 ..
+// 15: 30 words) in tensor memory: they are the same in every step, and read
+// from there they take none of the shared-memory pipe, the busiest of the
+// kernels with three CTAs per SM (14 of 72 wavefronts per input and spectrum).
+// `t` is the first of the 56 columns of the warp's lane quarter; warps w and
+// w + 4 share a quarter and hold the same tables. Written by warps 0 .. 3.
+constexpr uint32_t kTmTapCols = 24;
+
+template <int kW, bool kFpga> __device__ __forceinline__ void tm_tables(uint32_t t, const int *filter, int tid)
+{
+    int hc[2][kP];
+    load_taps(filter, 2 * (tid & 63), hc);
+    typename WolaTap<kW>::type tp[kP];
+    make_taps<kW, kFpga>(hc, tp);
+#pragma unroll
+    for (int p = 0; p < kP; p += 2) {
+        uint32_t w[4];
+        if constexpr (kW == kWolaInt32) {
+            w[0] = tp[p].x, w[1] = tp[p].y, w[2] = tp[p + 1].x, w[3] = tp[p + 1].y;
+        } else {
+            w[0] = __float_as_uint(tp[p].x), w[1] = __float_as_uint(tp[p].y);
+            w[2] = __float_as_uint(tp[p + 1].x), w[3] = __float_as_uint(tp[p + 1].y);
+        }
+        tmem_st4(t + 2 * p, w);
+    }
+#pragma unroll
+    for (int k1 = 1; k1 < 16; k1 += 2) { // the 32nd pair of columns is not read
+        const float2 a = w128((tid & 7) * k1), b = w128((tid & 7) * (k1 + 1));
+        const uint32_t w[4] = {__float_as_uint(a.x), __float_as_uint(a.y), __float_as_uint(b.x), __float_as_uint(b.y)};
+        tmem_st4(t + kTmTapCols + 2 * (k1 - 1), w);
+    }
+    tmem_wait_st();
+}
+
+template <int kW> __device__ __forceinline__ void tm_taps(uint32_t t, typename WolaTap<kW>::type (&tp)[kP])
+{
+    uint32_t a[16], b[8];
+    tmem_ld16(t, a);
+    tmem_ld8(t + 16, b);
+#pragma unroll
+    for (int p = 0; p < kP; p++) {
+        const uint32_t x = p < 8 ? a[2 * p] : b[2 * p - 16], y = p < 8 ? a[2 * p + 1] : b[2 * p - 15];
+        if constexpr (kW == kWolaInt32) tp[p] = make_int2((int)x, (int)y);
+        else tp[p] = make_float2(__uint_as_float(x), __uint_as_float(y));
+    }
+}
+
+template <bool kDemote, bool kScale>
+__device__ __forceinline__ void tm_fft_rows(float2 (*buf)[kFftRow], uint32_t t, int tid)
+{
+    fft_rows_with<kDemote, kScale>(buf, tid, [&](float2 *row, int j) {
+        fft128_pass1_with<-1>(row, j, [&](float2 (&x)[16]) {
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                uint32_t w[16];
+                tmem_ld16(t + kTmTapCols + 16 * h, w);
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (8 * h + i + 1 < 16)
+                        x[8 * h + i + 1] = cmul_tw<-1>(x[8 * h + i + 1], __uint_as_float(w[2 * i]), __uint_as_float(w[2 * i + 1]));
+            }
+        });
+    });
 }
 
 template <bool kDemote, bool kScale, int G>
@@ -394,15 +474,6 @@ template <int G> __device__ __forceinline__ void init_front(FrontSmemT<G> &sm, i
         mbar_init(&sm.bar[1], 1);
         fence_mbar_init();
     }
-}
-
-// Taps of samples n0, n0+1: h[K P - K p - n - 1] (pfb.cpp:159).
-__device__ __forceinline__ void load_taps(const int *filter, int n0, int (&hc)[2][kP])
-{
-#pragma unroll
-    for (int q = 0; q < 2; q++)
-#pragma unroll
-        for (int p = 0; p < kP; p++) hc[q][p] = __ldg(filter + kK * kP - kK * p - (n0 + q) - 1);
 }
 
 // The rows of input li are written by the WOLA and transformed by the FFT in
@@ -604,59 +675,65 @@ __global__ void __launch_bounds__(64 * G, G == 4 ? 2 : 1)
 // warps) with the same arithmetic in the same order (identical results):
 //   * each thread's 36 beam sums stay in tensor memory between steps
 //     (tcgen05.ld at the start of its beam phase, tcgen05.st at its end; one
-//     128-column allocation per CTA, warps w and w + 4 sharing a lane
-//     quarter at columns 0 and 64), so no register is held across steps;
-//   * the taps come from shared memory each step (12 loads per thread);
+//     128-column allocation per CTA), so no register is held across steps;
+//   * the taps and the FFT's twiddles come from tensor memory each step;
 //   * frames and weights are single-buffered: step it + 1's frames are copied
 //     as soon as every thread has finished step it's WOLA (the block barrier
 //     after the FFT) and land during its beam sums; step it's weights are
 //     copied after step it's first block barrier (every thread has finished
 //     step it - 1's sums) and land during its WOLA and FFT.
-// 72 KB of shared memory, at most 80 registers per thread.
-template <class Tap> struct TmSmem {
-    char2 stage[kG][kWin][kK];             // TMA destination: frames
+// 66 KB of shared memory, at most 80 registers per thread. The split sums take
+// two CTAs per SM with 126 registers and double-buffered frames instead.
+//
+// What bounds it: the shared-memory pipe (57 wavefronts per input and spectrum
+// of 102 clocks) and the FMA pipe (61) in turns, issue 65 %. Four channels'
+// second, FP32 / split / int32 sums / --smart: 3.42 / 3.59 / 3.82 / 4.00 ms;
+// with taps and twiddles in shared memory (72 wavefronts) 3.55 / 4.01 / 3.89 /
+// 4.09 ms, the two-CTA shape 3.55 / 3.80 / 4.04 / 4.05 ms. FP32 sums with two
+// CTAs per SM and double-buffered frames: 3.53 ms.
+template <int kStages> struct TmSmem {
+    char2 stage[kStages][kG][kWin][kK];    // TMA destination: frames
     float4 wst[2][kG / 2][kK];             // TMA destination: weights [row][tile][k']
     float2 buf[kG * kT][kFftRow];          // WOLA output -> FFT (in place) -> voltages
-    float2 tw[128];                        // W128 twiddles
-    Tap taps[kP][kK / 2];                  // per (tap, sample pair n0 / 2)
-    uint64_t bar_f, bar_w;
+    uint64_t bar_f[kStages], bar_w;
     uint32_t tmem;
 };
-static_assert(offsetof(TmSmem<float2>, wst) % 128 == 0 && offsetof(TmSmem<float2>, tw) % 16 == 0,
-              "TMA / vector alignment");
-constexpr uint32_t kTmCols = 128;          // TMEM columns per CTA (three CTAs: 384 of 512)
+static_assert(offsetof(TmSmem<1>, wst) % 128 == 0 && offsetof(TmSmem<1>, buf) % 16 == 0, "TMA / vector alignment");
+// TMEM columns per CTA (three CTAs: 384 of 512): the sums of warps w and w + 4
+// at 0 and 36, their tables at 72
+constexpr uint32_t kTmCols = 128, kTmTables = 72;
 
 // Frames of step `it` into the single stage: lane 0 of warp li (li < kG)
 // copies input it * kG + li, lane 0 of warp 0 posts the byte count first
 // (completing its own shortfall when frames fell outside the buffers, as
 // produce_spread does).
-template <class Tap>
-__device__ __forceinline__ void tm_frames(TmSmem<Tap> &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
+template <int T, int kStages>
+__device__ __forceinline__ void tm_frames(TmSmem<kStages> &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
                                           unsigned *status)
 {
     if ((threadIdx.x & 31) != 0) return;
     const int warp = threadIdx.x >> 5;
     if (warp >= kG) return;
-    const int w_end = min(m0 + kWin, nspectra + kP - 1);
+    const int w_end = min(m0 + T + kP - 1, nspectra + kP - 1);
     const uint32_t per_input = (w_end - m0) * kFrameBytes;
     if (warp == 0) {
         uint32_t total = 0;
         for (int li = 0; li < kG; li++)
             if (it * kG + li < vv.ninputs) total += per_input;
-        mbar_arrive_expect_tx(&sm.bar_f, total);
+        mbar_arrive_expect_tx(&sm.bar_f[it % kStages], total);
     }
     const int pos = it * kG + warp;
     if (pos < vv.ninputs) {
-        const uint32_t issued = issue_frames(vv, cc, pos, m0, w_end, sm.stage[warp][0], &sm.bar_f, status);
+        const uint32_t issued = issue_frames(vv, cc, pos, m0, w_end, sm.stage[it % kStages][warp][0], &sm.bar_f[it % kStages], status);
         if (issued != per_input)
-            asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.bar_f)),
+            asm volatile("mbarrier.complete_tx.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sm.bar_f[it % kStages])),
                          "r"(per_input - issued)
                          : "memory");
     }
 }
 
 // The two Jones rows of step `it`'s tiles, by lane 0 of warp kG.
-template <class Tap> __device__ __forceinline__ void tm_weights(TmSmem<Tap> &sm, const CUtensorMap *wmap, int cc, int it)
+template <int kStages> __device__ __forceinline__ void tm_weights(TmSmem<kStages> &sm, const CUtensorMap *wmap, int cc, int it)
 {
     if (threadIdx.x != 32 * kG) return;
     constexpr uint32_t kWBytes = (kG / 2) * kK * 16;
@@ -665,35 +742,28 @@ template <class Tap> __device__ __forceinline__ void tm_weights(TmSmem<Tap> &sm,
     tma_load_5d(sm.wst[1][0], wmap, 0, 1, 0, (kG / 2) * it, cc, &sm.bar_w);
 }
 
-template <int kW, bool kFpga, bool kDemote>
-__global__ void __launch_bounds__(kThreads, 3)
-    beam_tm_kernel(const BeamArgs a, const __grid_constant__ CUtensorMap wmap)
+// The split sums of all 8 spectra in one pass (19 frames widened once instead of
+// 30 in two passes) need more than 80 registers: two CTAs per SM, whose shared
+// memory leaves room for two steps' frames (one step's: 3.78 ms).
+constexpr int kTmPass = kT;
+template <int kW> constexpr int kTmStages = kW == kWolaSplit ? 2 : 1; // frames of how many steps
+
+// T: spectra of this CTA, as in beam_body.
+template <int kW, bool kFpga, bool kDemote, int T>
+__device__ __forceinline__ void beam_tm_body(const BeamArgs &a, const CUtensorMap *wmap, TmSmem<kTmStages<kW>> &sm, int cc, int m0)
 {
-    using Tap = typename WolaTap<kW>::type;
+    constexpr int kStages = kTmStages<kW>;
     constexpr int kTiles = kG / 2;       // tiles per step
     constexpr int kMh = kG / 2;          // threads per k' (spectra m = mh + kMh mi)
-    constexpr int kMi = kT / kMh;        // spectra per thread
-    static_assert(kMi * 9 == 36, "36 beam sums per thread");
-    extern __shared__ __align__(1024) unsigned char smem_raw[];
-    TmSmem<Tap> &sm = *reinterpret_cast<TmSmem<Tap> *>(smem_raw);
+    constexpr int kMi = T / kMh;         // spectra per thread
+    static_assert(T % kMh == 0 && kMi * 9 <= 36, "at most 36 beam sums per thread");
     const int tid = threadIdx.x, warp = tid >> 5;
-    const int cc = blockIdx.y;
-    const int m0 = blockIdx.x * kT;
     const int nsteps = (a.vv.ninputs + kG - 1) / kG;
     const int li = tid >> 6, n0 = 2 * (tid & 63);
 
-    if (tid == 0) prefetch_tmap(&wmap);
-    init_twiddles(sm.tw, tid);
-    if (tid < kK / 2) {
-        int hc[2][kP];
-        load_taps(a.filter, n0, hc);
-        Tap t[kP];
-        make_taps<kW, kFpga>(hc, t);
-#pragma unroll
-        for (int p = 0; p < kP; p++) sm.taps[p][tid] = t[p];
-    }
+    if (tid == 0) prefetch_tmap(wmap);
     if (tid == 0) {
-        mbar_init(&sm.bar_f, 1);
+        for (int i = 0; i < kStages; i++) mbar_init(&sm.bar_f[i], 1);
         mbar_init(&sm.bar_w, 1);
         fence_mbar_init();
     }
@@ -704,41 +774,46 @@ __global__ void __launch_bounds__(kThreads, 3)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    // this thread's 36 sums: lane 32 (warp % 4) + lane, columns 64 (warp / 4) ..
-    const uint32_t tacc = sm.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(64 * (warp >> 2));
+    // this thread's 36 sums and its tables: lane 32 (warp % 4) + lane
+    const uint32_t tlane = sm.tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    const uint32_t tacc = tlane + (uint32_t)(36 * (warp >> 2)), ttab = tlane + kTmTables;
     if (nsteps > 0) {
-        tm_frames(sm, a.vv, cc, 0, m0, a.nspectra, a.status);
-        tm_weights(sm, &wmap, cc, 0);
+        tm_frames<T>(sm, a.vv, cc, 0, m0, a.nspectra, a.status);
+        tm_weights(sm, wmap, cc, 0);
     }
+    if (warp < 4) tm_tables<kW, kFpga>(ttab, a.filter, tid);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
 
     const int kp = tid & (kK - 1), mh = tid >> 7;
     bool wbad = false;                   // a weights wait gave up (leave at the next step's barrier)
     int it = 0;
     for (; it < nsteps; it++) {
         // step it's frames have landed and every thread has finished step it - 1
-        const bool got = mbar_wait_bounded(&sm.bar_f, it & 1, 1u << 22);
+        const bool got = mbar_wait_bounded(&sm.bar_f[it % kStages], it / kStages & 1, 1u << 22);
         if (__syncthreads_or(!got || wbad)) break;
-        if (it > 0) tm_weights(sm, &wmap, cc, it);
+        if (it > 0) tm_weights(sm, wmap, cc, it);
+        if (kStages == 2 && it + 1 < nsteps) tm_frames<T>(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
         {
-            Tap t[kP];
-#pragma unroll
-            for (int p = 0; p < kP; p++) t[p] = sm.taps[p][tid & (kK / 2 - 1)];
-            wola_rows<kW, kFpga>(sm.stage[li][0], &sm.buf[li * kT], n0, t);
+            typename WolaTap<kW>::type t[kP];
+            tm_taps<kW>(ttab, t);
+            wola_rows<kW, kFpga, T, kTmPass>(sm.stage[it % kStages][li][0], &sm.buf[li * kT], n0, t);
         }
         input_barrier(li);
-        fft_rows<kDemote, kFpga>(sm.buf, sm.tw, tid);
+        if (T > kT / 2 || (warp & 1) * 4 < T) tm_fft_rows<kDemote, kFpga>(sm.buf, ttab, tid);
         __syncthreads();
         // every WOLA read of the stage is done: the next step's frames may land
-        if (it + 1 < nsteps) tm_frames(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
+        if (kStages == 1 && it + 1 < nsteps) tm_frames<T>(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
         if (!mbar_wait_bounded(&sm.bar_w, it & 1, 1u << 22)) {
             wbad = true;
             atomicOr(a.status, kErrWaitTimeout);
         }
         __syncwarp(); // the tensor-memory accesses are warp-collective
-        float acc[kMi * 9];
+        float acc[36];
         if (it == 0) {
 #pragma unroll
-            for (int q = 0; q < kMi * 9; q++) acc[q] = 0.f;
+            for (int q = 0; q < 36; q++) acc[q] = 0.f;
         } else {
             tmem_wait_st();
             tmem_ld36(tacc, acc);
@@ -763,17 +838,17 @@ __global__ void __launch_bounds__(kThreads, 3)
         // weights) get a bounded chance to land before the CTA exits
         if (tid == 0) {
             atomicOr(a.status, kErrWaitTimeout);
-            mbar_wait_bounded(&sm.bar_f, it & 1, 1u << 20);
+            mbar_wait_bounded(&sm.bar_f[it % kStages], it / kStages & 1, 1u << 20);
             if (it > 0) mbar_wait_bounded(&sm.bar_w, (it - 1) & 1, 1u << 20);
         }
     } else {
         // a weights copy whose wait gave up in the last step may still land
         if (tid == 0 && nsteps > 0) mbar_wait_bounded(&sm.bar_w, (nsteps - 1) & 1, 1u << 20);
         __syncwarp();
-        float acc[kMi * 9];
+        float acc[36];
         if (nsteps == 0) {
 #pragma unroll
-            for (int q = 0; q < kMi * 9; q++) acc[q] = 0.f;
+            for (int q = 0; q < 36; q++) acc[q] = 0.f;
         } else {
             tmem_wait_st();
             tmem_ld36(tacc, acc);
@@ -789,6 +864,18 @@ __global__ void __launch_bounds__(kThreads, 3)
     __syncthreads();
     tc_fence_after();
     if (warp == 0) tmem_dealloc(sm.tmem, kTmCols);
+}
+
+template <int kW, bool kFpga, bool kDemote, int kTail>
+__global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3)
+    beam_tm_kernel(const BeamArgs a, const __grid_constant__ CUtensorMap wmap)
+{
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    using Smem = TmSmem<kTmStages<kW>>;
+    Smem &sm = *reinterpret_cast<Smem *>(smem_raw);
+    const int b = blockIdx.x, n = a.ncc * a.n8;
+    if (b < n) beam_tm_body<kW, kFpga, kDemote, kT>(a, &wmap, sm, b / a.n8, b % a.n8 * kT);
+    else beam_tm_body<kW, kFpga, kDemote, kTail>(a, &wmap, sm, (b - n) / a.ntail, a.n8 * kT + (b - n) % a.ntail * kTail);
 }
 
 // ---------------------------------------------------------------------------
@@ -1008,20 +1095,19 @@ __device__ __forceinline__ double2 widen2(float x, float y)
 // output reads four inputs' values per half warp.
 constexpr int kPackRows = kT * kFftRow + 4;
 
-template <class Tap> struct PackSmem {
+struct PackSmem {
     char2 stage[kG][kWin][kK];             // TMA destination: frames
     float2 buf[kG][kPackRows];             // WOLA output -> FFT (in place) -> voltages
-    float2 tw[128];                        // W128 twiddles
-    Tap taps[kP][kK / 2];                  // per (tap, sample pair n0 / 2)
     uint64_t bar_f;
     uint32_t tmem;
 };
-static_assert(offsetof(PackSmem<float2>, tw) % 16 == 0 && offsetof(PackSmem<float2>, taps) % 16 == 0, "vector alignment");
+static_assert(offsetof(PackSmem, buf) % 16 == 0, "vector alignment");
+// TMEM columns: the waiting 4-bit words of warps w and w + 4 at 0 and 16, the tables at 32
+constexpr uint32_t kPackTables = 32;
 
 // Frames of step `it` into the single stage, input order[it * kG + li] by lane
 // 0 of warp li; lane 0 of warp 0 posts the byte count first.
-template <class Tap>
-__device__ __forceinline__ void pack_frames(PackSmem<Tap> &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
+__device__ __forceinline__ void pack_frames(PackSmem &sm, const VoltView &vv, int cc, int it, int m0, int nspectra,
                                             unsigned *status, const int *order)
 {
     if ((threadIdx.x & 31) != 0) return;
@@ -1045,20 +1131,19 @@ __device__ __forceinline__ void pack_frames(PackSmem<Tap> &sm, const VoltView &v
     }
 }
 
-// The beam kernels' front end at three CTAs per SM (taps from shared memory,
+// The beam kernels' front end at three CTAs per SM (tables from tensor memory,
 // frames single-buffered and copied while the step's rows are written out, at
 // most 80 registers; the split sums need 122, two CTAs) and the packing of its
 // rows. kDemote is the 4-bit output. Against two CTAs per SM with taps and
 // held words in registers, every column in one CTA and the instruction's
 // conversions: 10,000 spectra x 256 inputs to 4 bits with int32 sums 1,353 ->
-// 1,107 us (issue 69 %, FMA and ALU pipes 42 %), 4,000 spectra to complex
-// double 787 -> 578 us (shared-memory pipe 69 %, DRAM 50 %: 3.6 TB/s written).
+// 1,060 us (issue 70 %, FMA and ALU pipes 42 %), 4,000 spectra to complex
+// double 787 -> 565 us (shared-memory pipe 65 %, DRAM 50 %: 3.7 TB/s written).
 template <int kW, bool kFpga, bool kDemote>
 __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kernel(const PackArgs a)
 {
-    using Tap = typename WolaTap<kW>::type;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    PackSmem<Tap> &sm = *reinterpret_cast<PackSmem<Tap> *>(smem_raw);
+    PackSmem &sm = *reinterpret_cast<PackSmem *>(smem_raw);
     const int tid = threadIdx.x;
     const int cc = blockIdx.y;
     const int m0 = blockIdx.x * kT;
@@ -1071,23 +1156,14 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
     // (spectrum, channel) row: one 4-byte store in the 4-bit mode, 64
     // contiguous bytes in the complex-double mode. The per-input results do
     // not depend on the order.
-    int *inv = reinterpret_cast<int *>(smem_raw + sizeof(PackSmem<Tap>));
+    int *inv = reinterpret_cast<int *>(smem_raw + sizeof(PackSmem));
     for (int j = tid; j < I; j += kThreads) inv[j] = -1;
     __syncthreads();
     for (int i = tid; i < I; i += kThreads) {
         const int io = __ldg(a.i_idx + i);
         if (io >= 0 && io < I) inv[io] = i;
     }
-    init_twiddles(sm.tw, tid);
     const int li = tid >> 6, n0 = 2 * (tid & 63);
-    if (tid < kK / 2) {
-        int hc[2][kP];
-        load_taps(a.filter, n0, hc);
-        Tap t[kP];
-        make_taps<kW, kFpga>(hc, t);
-#pragma unroll
-        for (int p = 0; p < kP; p++) sm.taps[p][tid] = t[p];
-    }
     if (tid == 0) {
         mbar_init(&sm.bar_f, 1);
         fence_mbar_init();
@@ -1101,16 +1177,19 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
         if (tid == 0) atomicOr(a.status, kErrBadInput);
         return;
     }
-    if constexpr (kDemote) {
-        if (tid < 32) {
-            tmem_alloc(&sm.tmem, 32);
-            tmem_relinquish();
-        }
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
+    if (tid < 32) {
+        tmem_alloc(&sm.tmem, kTmCols);
+        tmem_relinquish();
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tlane = sm.tmem + ((uint32_t)(32 * ((tid >> 5) & 3)) << 16), ttab = tlane + kPackTables;
     pack_frames(sm, a.vv, cc, step0, m0, a.nspectra, a.status, inv);
+    if (tid < 128) tm_tables<kW, kFpga>(ttab, a.filter, tid);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
 
     const bool imag_first = (a.flags & VGB_PFB_IMAG_PART_FIRST) != 0;
     const int kp = tid & (kK - 1), mh = tid >> 7;
@@ -1118,7 +1197,7 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
     // spectra wait in tensor memory (column 4 (it & 3) + mi of its lane, warps
     // w and w + 4 at columns 0 and 16) and are written together every fourth
     // step; as registers they would be spilled
-    const uint32_t theld = kDemote ? sm.tmem + ((uint32_t)(32 * ((tid >> 5) & 3)) << 16) + (uint32_t)(16 * (tid >> 7)) : 0u;
+    const uint32_t theld = tlane + (uint32_t)(16 * (tid >> 7));
     int it = step0;
     for (; it < nsteps; it++) {
         const int phase = (it - step0) & 1;
@@ -1133,13 +1212,12 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
             break;
         }
         {
-            Tap t[kP];
-#pragma unroll
-            for (int p = 0; p < kP; p++) t[p] = sm.taps[p][tid & (kK / 2 - 1)];
-            wola_rows<kW, kFpga>(sm.stage[li][0], reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), n0, t);
+            typename WolaTap<kW>::type t[kP];
+            tm_taps<kW>(ttab, t);
+            wola_rows<kW, kFpga, kT, kTmPass>(sm.stage[li][0], reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), n0, t);
         }
         input_barrier(li);
-        fft_rows<kDemote, kFpga>(reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), sm.tw, tid & 63);
+        tm_fft_rows<kDemote, kFpga>(reinterpret_cast<float2(*)[kFftRow]>(sm.buf[li]), ttab, tid & 63);
         __syncthreads();
         // every WOLA read of the stage is done: the next step's frames may land
         if (it + 1 < nsteps) pack_frames(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status, inv);
@@ -1204,16 +1282,12 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
             }
         }
     }
-    if constexpr (kDemote) {
-        __syncwarp();
-        tmem_wait_st();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid < 32) tmem_dealloc(sm.tmem, 32);
-    } else if (it < nsteps) {
-        __syncthreads();
-    }
+    __syncwarp();
+    tmem_wait_st();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (tid < 32) tmem_dealloc(sm.tmem, kTmCols);
 }
 
 // ---------------------------------------------------------------------------
@@ -1258,14 +1332,14 @@ static int dispatch(const Args &a, dim3 grid, int wola, bool fpga, bool demote, 
 static std::atomic<int> g_pfb_variant{0}; // 0: autotuned; else the forced variant (3, 4, 5 or 8)
 static std::atomic<int> g_pfb_last{0};    // inputs per step of the last fused launch
 
-// Tiles of beam_kernel with `per_sm` CTAs per SM: whole waves of kT spectra per
-// CTA, and the spectra left over in tiles of 2 (`least` 2) or 4 where that fills
-// at most one more wave. A second of one channel is 1,250 tiles of 8 on 304
+// Tiles of a beam kernel with `per_sm` CTAs per SM: whole waves of kT spectra per
+// CTA, and the spectra left over in tiles of the smallest of least, least +
+// step, ... < kT spectra that fill at most one more wave, if any does. A second of one channel is 1,250 tiles of 8 on 304
 // places, 34 of them in a fifth wave: 4 x 304 tiles and 136 of 2 spectra take
 // 0.94 instead of 0.99 ms. A CTA of 2 spectra converts 13 frames for them and
 // takes about a third of a full one's time, so nothing else is split. Returns
 // the spectra of a leftover tile.
-static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least)
+static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least, int step)
 {
     static std::atomic<int> sms{0};
     if (!sms.load()) {
@@ -1282,7 +1356,7 @@ static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least)
     const long long full = total / (kT * slots) * slots; // tiles in whole waves
     const int n8 = (int)std::min<long long>(full / ncc, a.nspectra / kT);
     const int left = a.nspectra - n8 * kT;
-    for (int t = least; t < kT; t *= 2)
+    for (int t = least; t < kT; t += step)
         if (left > 0 && (long long)((left + t - 1) / t) * ncc <= slots) {
             a.n8 = n8;
             a.ntail = (left + t - 1) / t;
@@ -1290,7 +1364,7 @@ static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least)
         }
     a.n8 = (a.nspectra + kT - 1) / kT;
     a.ntail = 0;
-    return 4;
+    return least;
 }
 
 template <int A, bool B, bool C> struct BeamSel {
@@ -1301,8 +1375,10 @@ template <int A, bool B, bool C> struct BeamSel {
         if (rc) return rc;
         g_pfb_last = g;
         if (g == 5) {
-            auto kern = beam_tm_kernel<A, B, C>;
-            constexpr int kSmem = (int)sizeof(TmSmem<typename WolaTap<A>::type>);
+            BeamArgs b = a;
+            const int tail = beam_tiles(b, (int)grid.y, A == kWolaSplit ? 2 : 3, 4, 2);
+            auto kern = tail == 4 ? beam_tm_kernel<A, B, C, 4> : beam_tm_kernel<A, B, C, 6>;
+            constexpr int kSmem = (int)sizeof(TmSmem<kTmStages<A>>);
             if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem),
                                  "cudaFuncSetAttribute(tm smem)")))
                 return rc;
@@ -1310,7 +1386,7 @@ template <int A, bool B, bool C> struct BeamSel {
             if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, 100),
                                  "cudaFuncSetAttribute(tm carveout)")))
                 return rc;
-            kern<<<grid, kThreads, kSmem, st>>>(a, wmap);
+            kern<<<b.ncc * (b.n8 + b.ntail), kThreads, kSmem, st>>>(b, wmap);
         } else if (g == 3) {
             auto kern = beam_ws_kernel<A, B, C>;
             if ((rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1320,13 +1396,13 @@ template <int A, bool B, bool C> struct BeamSel {
             kern<<<grid, kWsThreads, sizeof(WsSmem), st>>>(a, wmap);
         } else if (g == 8) {
             BeamArgs b = a;
-            beam_tiles(b, (int)grid.y, 1, 4);
+            beam_tiles(b, (int)grid.y, 1, 4, 4);
             if ((rc = prep<8>(beam_kernel<A, B, C, 8, 4>))) return rc;
             beam_kernel<A, B, C, 8, 4><<<b.ncc * (b.n8 + b.ntail), 512, front_smem<8>(), st>>>(b, wmap);
         } else {
             BeamArgs b = a;
-            const int tail = beam_tiles(b, (int)grid.y, 2, 2);
-            auto kern = tail == 2 ? beam_kernel<A, B, C, 4, 2> : beam_kernel<A, B, C, 4, 4>;
+            beam_tiles(b, (int)grid.y, 2, 2, 6);
+            auto kern = beam_kernel<A, B, C, 4, 2>;
             if ((rc = prep<4>(kern))) return rc;
             kern<<<b.ncc * (b.n8 + b.ntail), 256, front_smem<4>(), st>>>(b, wmap);
         }
@@ -1384,7 +1460,7 @@ template <int A, bool B, bool C> struct BeamSel {
 template <int A, bool B, bool C> struct PackSel {
     static int run(const PackArgs &a, dim3 grid, cudaStream_t st)
     {
-        constexpr size_t base = sizeof(PackSmem<typename WolaTap<A>::type>);
+        constexpr size_t base = sizeof(PackSmem);
         int rc = check_cuda(cudaFuncSetAttribute(pack_kernel<A, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)(base + sizeof(int) * kPackMaxInputs)),
                             "cudaFuncSetAttribute(pack smem)");

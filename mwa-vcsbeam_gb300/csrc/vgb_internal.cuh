@@ -375,23 +375,32 @@ __device__ __forceinline__ float2 w128(int m) { return make_float2(__ldg(&kCos12
 // over q, twiddle by W128^{j k1} from `tw` (cos/sin pairs of the positive
 // angle 2*pi*j*k1/128 at fft128_tw_slot(k1, j)) and write back in place as
 // Y_j[k1].
-template <int SIGN>
-__device__ __forceinline__ void fft128_pass1(float2 *row, const float2 *tw, int j)
+// `twiddles(x)` multiplies x[k1] by W128^{j k1}.
+template <int SIGN, class Twiddles>
+__device__ __forceinline__ void fft128_pass1_with(float2 *row, int j, Twiddles &&twiddles)
 {
     float2 x[16];
 #pragma unroll
     for (int q = 0; q < 16; q++) x[q] = row[8 * q + j];
     __syncwarp();
     dft16<SIGN>(x);
-    const float4 *tw4 = reinterpret_cast<const float4 *>(tw);
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float4 w = tw4[i * 8 + j]; // W^{j 2i}, W^{j (2i + 1)}
-        if (i > 0) x[2 * i] = cmul_tw<SIGN>(x[2 * i], w.x, w.y);
-        x[2 * i + 1] = cmul_tw<SIGN>(x[2 * i + 1], w.z, w.w);
-    }
+    twiddles(x);
 #pragma unroll
     for (int k1 = 0; k1 < 16; k1++) row[k1 * 9 + j] = x[k1];
+}
+
+template <int SIGN>
+__device__ __forceinline__ void fft128_pass1(float2 *row, const float2 *tw, int j)
+{
+    fft128_pass1_with<SIGN>(row, j, [&](float2 (&x)[16]) {
+        const float4 *tw4 = reinterpret_cast<const float4 *>(tw);
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const float4 w = tw4[i * 8 + j]; // W^{j 2i}, W^{j (2i + 1)}
+            if (i > 0) x[2 * i] = cmul_tw<SIGN>(x[2 * i], w.x, w.y);
+            x[2 * i + 1] = cmul_tw<SIGN>(x[2 * i + 1], w.z, w.w);
+        }
+    });
 }
 
 // Pass 2: thread t of the group produces X[k1 + 16 k2] for k1 = t, t + 8 and
