@@ -168,6 +168,7 @@ struct MbWeightArgs {
     float *Q32;           //                    Q [nfine][Mq][4A]
     MbStats stats;        // reset here for the run's rows
     int B;
+    int per_block;        // beams of a block (mb_weights_pair_kernel)
 };
 
 __device__ __forceinline__ float2 cmul32(float2 a, float2 b)
@@ -240,7 +241,7 @@ __device__ __forceinline__ float from_bits(uint16_t b, bool fp16)
 // embedded weights (hi, lo planes) and the scaled, split Q rows.
 constexpr int kMbWeightThreads = 128;
 constexpr int kMbPairMaxTiles = 512; // arrays the pair kernel covers (2 tiles per thread, 256 threads)
-constexpr int kMbWeightBeams = 8;    // beams per block in the pair kernel
+constexpr int kMbWeightBeams = 8;    // beams per block in the pair kernel, at most
 
 // Phase (cos, sin) of tile a for beam p at frequency f: turns dt * f in FP64,
 // wrapped to [-1/2, 1/2], then sin/cos in FP32.
@@ -408,8 +409,8 @@ __global__ void __launch_bounds__(256, 4) mb_weights_pair_kernel(const MbWeightA
     }
     const double f = (double)(uint32_t)w.freq[c];
     const bool h16 = w.fp16 != 0;
-    const int p_end = min(w.Bp, ((int)blockIdx.x + 1) * kMbWeightBeams);
-    for (int p = blockIdx.x * kMbWeightBeams; p < p_end; p++) {
+    const int p_end = min(w.B, ((int)blockIdx.x + 1) * w.per_block);
+    for (int p = blockIdx.x * w.per_block; p < p_end; p++) {
         mb_reset_stats(w, c, p);
         float mx[4] = {0.f, 0.f, 0.f, 0.f};
         float2 J[2][4];
@@ -549,6 +550,89 @@ __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
     }
 }
 
+// The same for one beam tile (at most 32 beams): there V is read once, and the wide
+// copy's write and read were most of such a run. V keeps the input's own values
+// instead, gathered to tile order, [c][s][tile]{Q, P} bytes (8-bit: qr, qi, pr, pi;
+// 4-bit: the two bytes as they came), and mb_beam_few_kernel widens them on the way
+// to its MMAs. C is the same integers (dp4a; 4-bit values as 16 x, products 256 x).
+// Thread: one tile (8-bit) or two (4-bit), 4 bytes a sample. Bound by memory: 8-bit,
+// 128 tiles, 1.57 GB in 226 us, 85 % of the DRAM pipe (mb_convert_kernel 2.23 GB, 390 us).
+template <bool kInt8> __global__ void __launch_bounds__(128) mb_gather_voltages_kernel(const MbConvArgs g)
+{
+    constexpr int kT = kInt8 ? 1 : 2;
+    extern __shared__ uint4 conv_smem[];
+    const uint8_t *rows = reinterpret_cast<const uint8_t *>(conv_smem);
+    const int c = blockIdx.x, t = blockIdx.y;
+    const int rowbytes = g.ni * (kInt8 ? 2 : 1);
+    const int per_row = rowbytes / 16;
+    for (int e = threadIdx.x; e < kMbInt * per_row; e += blockDim.x) {
+        const int k = e / per_row, i = e - k * per_row;
+        const uint4 *src = reinterpret_cast<const uint4 *>(g.v + ((long long)(t * kMbInt + k) * g.nfine + c) * rowbytes) + i;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(&conv_smem[e])), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    const int units = g.A / kT;
+    for (int u = threadIdx.x; u < units; u += blockDim.x) {
+        uint32_t iq[kT], ip[kT];
+        bool bad = false;
+#pragma unroll
+        for (int j = 0; j < kT; j++) {
+            iq[j] = g.polQ[kT * u + j];
+            ip[j] = g.polP[kT * u + j];
+            bad |= iq[j] >= (uint32_t)g.ni || ip[j] >= (uint32_t)g.ni;
+        }
+        if (bad) {
+            atomicOr(g.status, kErrBadInput);
+            continue;
+        }
+        int cqq[kT] = {}, cpp[kT] = {}, cr[kT] = {}, cqp[kT] = {}, cpq[kT] = {};
+        uint32_t *out = reinterpret_cast<uint32_t *>(g.V) + ((long long)c * g.ns + t * kMbInt) * units + u;
+#pragma unroll
+        for (int k = 0; k < kMbInt; k++) {
+            const uint8_t *r = rows + k * rowbytes;
+            uint32_t o = 0;
+#pragma unroll
+            for (int j = 0; j < kT; j++) {
+                uint32_t Q, P; // bytes (re, im); 4-bit values in the high nibbles
+                if constexpr (kInt8) {
+                    Q = reinterpret_cast<const uint16_t *>(r)[iq[j]];
+                    P = reinterpret_cast<const uint16_t *>(r)[ip[j]];
+                    o = Q | (P << 16);
+                } else {
+                    const uint32_t bq = r[iq[j]], bp = r[ip[j]];
+                    o |= (bq | (bp << 8)) << (16 * j);
+                    Q = (bq & 0xF0u) | ((bq & 0xFu) << 12);
+                    P = (bp & 0xF0u) | ((bp & 0xFu) << 12);
+                }
+                const uint32_t Ps = __byte_perm(P, 0u, 0x4401); // (im, re)
+                cqq[j] = __dp4a((int)Q, (int)Q, cqq[j]);
+                cpp[j] = __dp4a((int)P, (int)P, cpp[j]);
+                cr[j] = __dp4a((int)Q, (int)P, cr[j]);
+                cqp[j] = __dp4a((int)(Q & 0xFF00u), (int)Ps, cqp[j]); // qi pr
+                cpq[j] = __dp4a((int)(Q & 0xFFu), (int)Ps, cpq[j]);   // qr pi
+            }
+            out[(long long)k * units] = o;
+        }
+#pragma unroll
+        for (int j = 0; j < kT; j++) {
+            constexpr int kShift = kInt8 ? 0 : 8;
+            const int cv[4] = {cqq[j] >> kShift, cpp[j] >> kShift, cr[j] >> kShift, (cqp[j] - cpq[j]) >> kShift};
+            uint16_t hi[4], lo[4];
+            for (int i = 0; i < 4; i++) {
+                const __half h = __float2half_rn((float)cv[i]);
+                hi[i] = __half_as_ushort(h);
+                lo[i] = __half_as_ushort(__float2half_rn((float)(cv[i] - (int)__half2float(h))));
+            }
+            __half *row = g.C + ((long long)c * g.nint_p + t) * g.Kb + 4 * (kT * u + j);
+            *reinterpret_cast<uint2 *>(row) = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
+            if (kInt8)
+                *reinterpret_cast<uint2 *>(row + 4 * g.A) =
+                    make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // The beam GEMM (persistent, one CTA per SM)
 // ---------------------------------------------------------------------------
@@ -619,49 +703,65 @@ __device__ __forceinline__ bool mb_epilogue_tile(const MbBeamArgs &g, uint32_t t
         return false;
     }
     tc_fence_after();
-    float sq = 0.f, pb = 0.f, pc = 0.f;
+    auto emit = [&](int ti, float val) {
+        if (writer && ti < nv) {
+            const float sv = g.invw * (val - qs * rv[ti - kI0]);
+            srow[ti] = sv;
+            smin = fminf(smin, sv);
+            smax = fmaxf(smax, sv);
+            if (kI0 == 0 && ti == 0 && t0 == 0) g.stats.nan0[((long long)c * g.B + p) * kNst + st] = sv != sv;
+        }
+    };
+    if constexpr (kNst == 4) {
+        // two integrations at a time: the cross terms of the first in lanes 0, 1 of a beam, of the
+        // second in lanes 2, 3 (the same products of the same pairs, 29 shuffles for 54)
+        const bool hi = l >= 2;
 #pragma unroll
-    for (int j = kC0 / 32; j <= (kC1 - 1) / 32; j++) {
-        float v[32];
-        tmem_ld32(tacc + 32 * j, v);
+        for (int i = kI0; i < kI1; i += 2) {
+            const bool two = i + 1 < kI1;
+            float x[20];
+            if (two) tmem_ld20(tacc + kMbInt * i, x);
+            else tmem_ld10(tacc + kMbInt * i, x);
+            float sa = 0.f, sb = 0.f, pb = 0.f, pc = 0.f;
 #pragma unroll
-        for (int col = 0; col < 32; col++) {
-            const int gcol = 32 * j + col;
-            if (gcol >= kC0 && gcol < kC1) {
-                const float x = v[col];
-                sq = fmaf(x, x, sq);
-                if (kNst == 4) {
-                    const float xb = __shfl_xor_sync(0xffffffffu, x, 2);
-                    const float xc = __shfl_xor_sync(0xffffffffu, x, 3);
-                    pb = fmaf(x, xb, pb);
-                    pc = fmaf(x, xc, pc);
-                }
-                if (gcol % kMbInt == kMbInt - 1) {
-                    const int ti = gcol / kMbInt;
-                    float val;
-                    if (kNst == 4) {
-                        // lanes of a beam: 0 Xr, 1 Xi, 2 Yr, 3 Yi
-                        const float t1 = sq + __shfl_xor_sync(0xffffffffu, sq, 1);
-                        const float t1o = __shfl_xor_sync(0xffffffffu, t1, 2);
-                        const float xx = l < 2 ? t1 : t1o, yy = l < 2 ? t1o : t1;
-                        const float re = pb + __shfl_xor_sync(0xffffffffu, pb, 1);
-                        const float d = __shfl_xor_sync(0xffffffffu, pc, 1) - pc;
-                        const float im = (l == 0 || l == 3) ? d : -d;
-                        val = l == 0 ? xx + yy : l == 1 ? xx - yy : l == 2 ? 2.f * re : -2.f * im;
-                    } else {
+            for (int k = 0; k < kMbInt; k++) {
+                const float xa = x[k], xb = x[two ? kMbInt + k : k];
+                sa = fmaf(xa, xa, sa);
+                sb = fmaf(xb, xb, sb);
+                const float own = hi ? xb : xa, other = hi ? xa : xb;
+                pb = fmaf(own, __shfl_xor_sync(0xffffffffu, other, 2), pb);
+                pc = fmaf(own, __shfl_xor_sync(0xffffffffu, other, 3), pc);
+            }
+            // lanes of a beam: 0 Xr, 1 Xi, 2 Yr, 3 Yi
+            const float re = pb + __shfl_xor_sync(0xffffffffu, pb, 1);
+            const float d = __shfl_xor_sync(0xffffffffu, pc, 1) - pc;
+            const float im = (l == 0 || l == 3) ? d : -d;
+            const float z = (l & 1) ? im : re, zo = __shfl_xor_sync(0xffffffffu, z, 2);
+#pragma unroll
+            for (int u = 0; u < (two ? 2 : 1); u++) {
+                const float sq = u ? sb : sa, zu = u ? z : zo;
+                const float t1 = sq + __shfl_xor_sync(0xffffffffu, sq, 1);
+                const float t1o = __shfl_xor_sync(0xffffffffu, t1, 2);
+                emit(i + u, l == 0 ? t1 + t1o : l == 1 ? t1 - t1o : l == 2 ? 2.f * zu : -2.f * zu);
+            }
+        }
+    } else {
+        float sq = 0.f;
+#pragma unroll
+        for (int j = kC0 / 32; j <= (kC1 - 1) / 32; j++) {
+            float v[32];
+            tmem_ld32(tacc + 32 * j, v);
+#pragma unroll
+            for (int col = 0; col < 32; col++) {
+                const int gcol = 32 * j + col;
+                if (gcol >= kC0 && gcol < kC1) {
+                    sq = fmaf(v[col], v[col], sq);
+                    if (gcol % kMbInt == kMbInt - 1) {
                         float t1 = sq + __shfl_xor_sync(0xffffffffu, sq, 1);
                         t1 += __shfl_xor_sync(0xffffffffu, t1, 2);
-                        val = t1;
+                        emit(gcol / kMbInt, t1);
+                        sq = 0.f;
                     }
-                    if (writer && ti < nv) {
-                        const float sv = g.invw * (val - qs * rv[ti - kI0]);
-                        srow[ti] = sv;
-                        smin = fminf(smin, sv);
-                        smax = fmaxf(smax, sv);
-                        if (kI0 == 0 && ti == 0 && t0 == 0)
-                            g.stats.nan0[((long long)c * g.B + p) * kNst + st] = sv != sv;
-                    }
-                    sq = pb = pc = 0.f;
                 }
             }
         }
@@ -813,6 +913,294 @@ __global__ void __launch_bounds__(kMbThreads, 1)
                     if (lane == 0) mbar_arrive(&sm.tempty[buf]);
                 });
             if (!ok) break;
+        }
+    }
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------------------
+// The beam GEMM for one beam tile (at most 32 beams)
+// ---------------------------------------------------------------------------
+// mb_beam_kernel's tile, products and epilogue (same order, same bits) from the
+// gathered voltages of mb_gather_voltages_kernel. With one beam tile the run was
+// bound by the 16-bit V going out to memory and back; this kernel reads a half
+// (8-bit) or a quarter (4-bit) of those bytes, and eight more warps widen each
+// step's 256 samples x 16 tiles into the 128-byte-swizzled operand. It is now bound
+// by the shared-memory pipe (per 64-wide K step, in 128-byte turns: MMA operands
+// 384 a plane, weights 128 a plane, voltages in 64 or 128, read 64 or 128, written
+// 256; epilogue shuffles 160 with four Stokes) and by the latency of the weights
+// from L2. 20 beams, 128 tiles, 10^4 samples, before -> now in us:
+//                              conversion   beam GEMM   coarse channel
+//   8-bit, FP16, Stokes I      390 -> 228   207 -> 182   718 -> 504
+//   4-bit, split, four Stokes  298 -> 166   236 -> 244   644 -> 493
+//   8-bit, split, four Stokes  392 -> 230   231 -> 260   775 -> 612
+// (with the shorter weights and byte stages). From two beam tiles on every tile would
+// widen the voltages again, on a pipe that is full with one: they keep the 16-bit V.
+//   warp 0 lane 0: TMA producer of the weight and voltage rings
+//   warp 1 lane 0: MMA issuer, once a step's weights have landed and its four
+//     widening warps have arrived
+//   warps 2..9: epilogue; warps 10..17: widening, two groups taking steps in turn
+// Every wait is bounded.
+constexpr int kMbFewEpi = 8;                        // epilogue warps, two per TMEM lane quarter
+constexpr int kMbWiden = 4, kMbWidenGroups = 2;     // widening warps of a step; groups taking steps in turn
+constexpr int kMbFewThreads = 64 + 32 * (kMbFewEpi + kMbWiden * kMbWidenGroups);
+
+// 224 KB of rings. Most in flight where the time went: weight steps for one plane
+// (3 -> 4: 200 -> 182 us), widened operands for two (2 -> 3: 301 -> 272 us with
+// 4-bit voltages), but not at the price of two steps of 8-bit voltages (283 -> 328).
+template <int kPlanes, bool kInt8> struct MbFewRing {
+    static constexpr int kTileA = 128 * 128;
+    static constexpr int kTileB = kMbN * 128;
+    static constexpr int kV = kPlanes == 2 && kInt8 ? 2 : 3; // widened operands
+    static constexpr int kW = kPlanes == 2 ? 3 : 4;          // weight steps
+    static constexpr int kStep = kMbN * (kInt8 ? 64 : 32);   // gathered voltages of 16 tiles
+    static constexpr int kP = (224 * 1024 - kV * kTileB - kW * kPlanes * kTileA) / kStep;
+};
+
+template <int kPlanes, bool kInt8> struct MbFewSmem {
+    using R = MbFewRing<kPlanes, kInt8>;
+    uint8_t v[R::kV][R::kTileB];
+    uint8_t w[R::kW][kPlanes * R::kTileA];
+    uint8_t packed[R::kP][R::kStep];
+    uint64_t vfull[R::kV], vempty[R::kV], wfull[R::kW], wempty[R::kW], pfull[R::kP], pempty[R::kP];
+    uint64_t tfull[2], tempty[2], drain;
+    uint32_t tmem;
+};
+
+template <bool kF16> __device__ __forceinline__ uint32_t mb_sub2(uint32_t x, uint32_t off)
+{
+    uint32_t r;
+    if (kF16) asm("sub.f16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(off));
+    else asm("sub.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(x), "r"(off));
+    return r;
+}
+
+// Four 8-bit values -> four 16-bit floats, exactly (u = x + 128 under 1024 in fp16,
+// under 2^23 in FP32 for bf16, whose upper half is the whole value).
+template <bool kF16> __device__ __forceinline__ uint2 mb_widen8(uint32_t w)
+{
+    w ^= 0x80808080u;
+    if constexpr (kF16) {
+        return make_uint2(mb_sub2<kF16>(__byte_perm(w, 0x64646464u, 0x4140), 0x64806480u),
+                          mb_sub2<kF16>(__byte_perm(w, 0x64646464u, 0x4342), 0x64806480u));
+    } else {
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) f[i] = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440 + i)) - 8388736.f;
+        return make_uint2(__byte_perm(__float_as_uint(f[0]), __float_as_uint(f[1]), 0x7632),
+                          __byte_perm(__float_as_uint(f[2]), __float_as_uint(f[3]), 0x7632));
+    }
+}
+
+// One 4+4-bit byte (high nibble first) -> two 16-bit floats, exactly (x + 8 under 128
+// in bf16, under 1024 in fp16).
+template <bool kF16> __device__ __forceinline__ uint32_t mb_widen4(uint32_t b)
+{
+    const uint32_t x = (b * 0x100001u) >> 4;
+    return mb_sub2<kF16>((x & 0x000F000Fu) ^ (kF16 ? 0x64086408u : 0x43084308u), kF16 ? 0x64086408u : 0x43084308u);
+}
+
+template <int kPlanes, bool kF16, int kNst, bool kInt8>
+__global__ void __launch_bounds__(kMbFewThreads, 1)
+    mb_beam_few_kernel(const __grid_constant__ CUtensorMap tw, const __grid_constant__ CUtensorMap tp, const MbBeamArgs g)
+{
+    using Ring = MbFewRing<kPlanes, kInt8>;
+    using Smem = MbFewSmem<kPlanes, kInt8>;
+    constexpr int kV = Ring::kV, kW = Ring::kW, kP = Ring::kP;
+    extern __shared__ uint8_t mb_raw[];
+    Smem &sm = *reinterpret_cast<Smem *>((reinterpret_cast<uintptr_t>(mb_raw) + 1023) & ~uintptr_t(1023));
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        prefetch_tmap(&tw);
+        prefetch_tmap(&tp);
+    }
+    if (warp == 0) {
+        // one lane to each kind and slot of barrier
+        if (lane < kV) {
+            mbar_init(&sm.vfull[lane], kMbWiden);
+            mbar_init(&sm.vempty[lane], 1);
+        }
+        if (lane < kW) {
+            mbar_init(&sm.wfull[lane], 1);
+            mbar_init(&sm.wempty[lane], 1);
+        }
+        if (lane < kP) {
+            mbar_init(&sm.pfull[lane], 1);
+            mbar_init(&sm.pempty[lane], kMbWiden);
+        }
+        if (lane < 2) {
+            mbar_init(&sm.tfull[lane], 1);
+            mbar_init(&sm.tempty[lane], kMbFewEpi);
+        }
+        if (lane == 2) mbar_init(&sm.drain, 1);
+        fence_mbar_init();
+    }
+    __syncwarp();
+    if (warp == 0) {
+        tmem_alloc(&sm.tmem, 512);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = sm.tmem;
+    // this CTA's tiles blockIdx.x + j gridDim.x (nfine ntn tiles fit 32 bits: 4096 x 2622), nk steps each
+    const uint32_t ntiles = ((uint32_t)g.total - blockIdx.x + gridDim.x - 1) / gridDim.x;
+    const uint32_t steps = ntiles * (uint32_t)g.nk;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // ---- TMA producer ----
+            bool ok = true;
+            uint32_t nw = 0, np = 0; // steps whose weights / voltages have been issued
+            auto weights = [&] {
+                const uint32_t s = nw % kW, r = nw / kW;
+                if (r > 0 && !mbar_wait_bounded(&sm.wempty[s], (r - 1) & 1, kMbPolls)) {
+                    ok = false;
+                    return;
+                }
+                const int c = (int)((blockIdx.x + nw / g.nk * gridDim.x) / g.ntn), kc = (int)(nw % g.nk);
+                mbar_arrive_expect_tx(&sm.wfull[s], kPlanes * Ring::kTileA);
+                tma_load_2d(sm.w[s], &tw, kc * 64, c * g.Mrows, &sm.wfull[s]);
+                if (kPlanes == 2)
+                    tma_load_2d(sm.w[s] + Ring::kTileA, &tw, kc * 64, (c + g.nfine) * g.Mrows, &sm.wfull[s]);
+                nw++;
+            };
+            auto voltages = [&] {
+                const uint32_t s = np % kP, r = np / kP;
+                if (r > 0 && !mbar_wait_bounded(&sm.pempty[s], (r - 1) & 1, kMbPolls)) {
+                    ok = false;
+                    return;
+                }
+                const uint32_t tile = blockIdx.x + np / g.nk * gridDim.x;
+                const int n = (int)(tile % g.ntn), c = (int)(tile / g.ntn), kc = (int)(np % g.nk);
+                mbar_arrive_expect_tx(&sm.pfull[s], Ring::kStep);
+                tma_load_2d(sm.packed[s], &tp, kc * (Ring::kStep / kMbN), c * g.ns + n * kMbUsed, &sm.pfull[s]);
+                np++;
+            };
+            // the voltages a whole ring ahead, the weights one step less: in turn, voltages j + kP wait
+            // for the widening of step j and weights j + kW - 1 for the products of step j - 1
+            while (np < kP && np < steps) voltages();
+            while (nw + 1 < kW && nw < steps) weights();
+            while (ok && (nw < steps || np < steps)) {
+                if (np < steps) voltages();
+                if (ok && nw < steps) weights();
+            }
+            if (!ok) atomicOr(g.status, kErrWaitTimeout);
+            // every load issued must have landed before the CTA leaves
+            for (uint32_t k = np > kP ? np - kP : 0; k < np; k++)
+                mbar_wait_bounded(&sm.pfull[k % kP], (k / kP) & 1, kMbPolls);
+            for (uint32_t k = nw > kW ? nw - kW : 0; k < nw; k++)
+                mbar_wait_bounded(&sm.wfull[k % kW], (k / kW) & 1, kMbPolls);
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // ---- MMA issuer ----
+            const uint32_t idesc = idesc_bf16_f32(kMbN, false, kF16);
+            uint32_t it = 0;
+            bool ok = true;
+            for (uint32_t tc = 0; tc < ntiles && ok; tc++) {
+                const int buf = tc & 1;
+                const uint32_t u = tc >> 1;
+                if (u > 0 && !mbar_wait_bounded(&sm.tempty[buf], (u - 1) & 1, kMbPolls)) {
+                    atomicOr(g.status, kErrWaitTimeout);
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t d = tmem + buf * kMbN;
+                for (int kc = 0; kc < g.nk; kc++, it++) {
+                    const uint32_t sv = it % kV, sw = it % kW;
+                    if (!mbar_wait_bounded(&sm.wfull[sw], (it / kW) & 1, kMbPolls) ||
+                        !mbar_wait_bounded(&sm.vfull[sv], (it / kV) & 1, kMbPolls)) {
+                        atomicOr(g.status, kErrWaitTimeout);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t sa = smem_u32(sm.w[sw]);
+                    const uint64_t a0 = sdesc_sw128(sa);
+                    const uint64_t a1 = sdesc_sw128(sa + Ring::kTileA);
+                    const uint64_t bd = sdesc_sw128(smem_u32(sm.v[sv]));
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        tc_mma(d, sdesc_advance_k(a0, k), sdesc_advance_k(bd, k), idesc, (kc | k) != 0);
+                        if (kPlanes == 2) tc_mma(d, sdesc_advance_k(a1, k), sdesc_advance_k(bd, k), idesc, 1);
+                    }
+                    tc_commit(&sm.vempty[sv]);
+                    tc_commit(&sm.wempty[sw]);
+                }
+                if (ok) tc_commit(&sm.tfull[buf]);
+            }
+            // all MMAs this thread issued have completed before teardown
+            tc_commit(&sm.drain);
+            mbar_wait_bounded(&sm.drain, 0, kMbPolls);
+        }
+    } else if (warp < 2 + kMbFewEpi) {
+        // ---- epilogue (mb_beam_kernel's, the 25 integrations in two ranges) ----
+        const int q4 = warp & 3;
+        for (uint32_t tc = 0; tc < ntiles; tc++) {
+            const int buf = tc & 1;
+            const uint32_t tile = blockIdx.x + tc * gridDim.x;
+            const uint32_t tacc = tmem + ((uint32_t)(32 * q4) << 16) + buf * kMbN;
+            const int n = (int)(tile % g.ntn), c = (int)(tile / g.ntn), row = 32 * q4 + lane;
+            auto wait = [&] { return mbar_wait_bounded(&sm.tfull[buf], (tc >> 1) & 1, kMbPolls); };
+            auto release = [&] {
+                if (lane == 0) mbar_arrive(&sm.tempty[buf]);
+            };
+            const bool ok = warp < 6 ? mb_epilogue_tile<kNst, 0, kMbNint / 2>(g, tacc, 0, n, c, row, wait, release)
+                                     : mb_epilogue_tile<kNst, kMbNint / 2, kMbNint>(g, tacc, 0, n, c, row, wait, release);
+            if (!ok) break;
+        }
+    } else {
+        // ---- widening: 16 bytes in (8-bit: 4 tiles of a sample, 4-bit: 8), 32 or 64 out, to the
+        // swizzled 16-byte pieces; every access covers all banks once ----
+        const int tid = (threadIdx.x - 32 * (2 + kMbFewEpi)) % (32 * kMbWiden);
+        for (uint32_t it = (warp - 2 - kMbFewEpi) / kMbWiden; it < steps; it += kMbWidenGroups) {
+            const uint32_t s = it % kV, r = it / kV, ps = it % kP;
+            if (!mbar_wait_bounded(&sm.pfull[ps], (it / kP) & 1, kMbPolls) ||
+                (r > 0 && !mbar_wait_bounded(&sm.vempty[s], (r - 1) & 1, kMbPolls))) {
+                if (lane == 0) atomicOr(g.status, kErrWaitTimeout);
+                break;
+            }
+            const uint4 *in = reinterpret_cast<const uint4 *>(sm.packed[ps]);
+            uint8_t *out = sm.v[s];
+            if constexpr (kInt8) {
+#pragma unroll 4
+                for (int u = tid; u < kMbN * 4; u += 32 * kMbWiden) {
+                    const uint4 w = in[u];
+                    const int row = u >> 2, ch = 2 * (u & 3);
+                    const uint2 a = mb_widen8<kF16>(w.x), b = mb_widen8<kF16>(w.y), c = mb_widen8<kF16>(w.z),
+                                d = mb_widen8<kF16>(w.w);
+                    *reinterpret_cast<uint4 *>(out + row * 128 + ((ch ^ (row & 7)) << 4)) = make_uint4(a.x, a.y, b.x, b.y);
+                    *reinterpret_cast<uint4 *>(out + row * 128 + (((ch + 1) ^ (row & 7)) << 4)) =
+                        make_uint4(c.x, c.y, d.x, d.y);
+                }
+            } else {
+#pragma unroll
+                for (int u = tid; u < kMbN * 2; u += 32 * kMbWiden) {
+                    const uint4 w = in[u];
+                    const int row = u >> 1, ch = 4 * (u & 1);
+                    const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const uint32_t x = ws[j];
+                        *reinterpret_cast<uint4 *>(out + row * 128 + (((ch + j) ^ (row & 7)) << 4)) =
+                            make_uint4(mb_widen4<kF16>(x & 0xFFu), mb_widen4<kF16>((x >> 8) & 0xFFu),
+                                       mb_widen4<kF16>((x >> 16) & 0xFFu), mb_widen4<kF16>(x >> 24));
+                    }
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the MMA reads these through the async proxy
+            __syncwarp();
+            if (lane == 0) {
+                mbar_arrive(&sm.pempty[ps]);
+                mbar_arrive(&sm.vfull[s]);
+            }
         }
     }
     __syncwarp();
@@ -1203,7 +1591,8 @@ struct MbRenormArgs {
 
 constexpr int kRnT = 128; // integrations per transpose chunk
 
-// Block: (32 channels, one beam and Stokes parameter). The row extremes come
+// Block: (32 channels, one beam and Stokes parameter, a share of the integrations
+// where that alone would leave SMs idle: 20 beams x 128 channels x 1000: 18 us in one share, 10 in 8). The row extremes come
 // from the beam epilogue (MbStats); one pass then quantises 128 integrations
 // at a time, packs four channels' bytes into a word, transposes in shared
 // memory and writes 16-byte runs of channels.
@@ -1229,7 +1618,7 @@ __global__ void __launch_bounds__(256, 4) mb_renorm_kernel(const MbRenormArgs a)
         const float scale = (float)((double)(mx - mn) / 256.0);
         s_off[threadIdx.x] = mn;
         s_scl[threadIdx.x] = scale;
-        if (c < a.nfine) {
+        if (c < a.nfine && blockIdx.z == 0) {
             const long long si = ((long long)p * a.nst + st) * a.nfine + c;
             a.scales[si] = scale;
             a.offsets[si] = mn;
@@ -1247,7 +1636,7 @@ __global__ void __launch_bounds__(256, 4) mb_renorm_kernel(const MbRenormArgs a)
     const float4 rcp = make_float4(1.f / scl.x, 1.f / scl.y, 1.f / scl.z, 1.f / scl.w);
     const bool wide = ((a.out_s | a.out_st | a.out_p) & 15) == 0 &&
                       (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && c0 + 32 <= a.nfine;
-    for (int t0 = 0; t0 < a.nint; t0 += kRnT) {
+    for (int t0 = blockIdx.z * kRnT; t0 < a.nint; t0 += gridDim.z * kRnT) {
         float e[4][4];
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -1297,6 +1686,7 @@ struct vgb_multibeam {
     float *d_Q32 = nullptr;
     uint32_t *d_stats = nullptr; // min keys, max keys, first-is-NaN: 3 x [nfine][B][nst]
     bool simt = false;
+    bool few = false;            // one beam tile on the tensor path: gathered voltages, mb_beam_few_kernel
     CUtensorMap tmW, tmV;
     CUtensorMap tmV2;            // voltages in 128-sample boxes: the pair kernel's half tiles
     int pair_clusters = -1;      // co-resident 2-CTA clusters of the pair kernel (-1: not yet asked)
@@ -1438,12 +1828,30 @@ int mb_pick_beam(vgb_multibeam *mb, const MbBeamArgs &a, cudaStream_t st)
     return rc;
 }
 
+template <int kPlanes, bool kF16, int kNst>
+int mb_launch_beam_few(vgb_multibeam *mb, const MbBeamArgs &a, cudaStream_t st)
+{
+    auto go = [&](auto kern, int smem) {
+        int rc = check_cuda(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
+                            "cudaFuncSetAttribute(mb_beam_few_kernel)");
+        if (!rc) kern<<<(unsigned)std::min<long long>(a.total, mb->nsm), kMbFewThreads, smem, st>>>(mb->tmW, mb->tmV, a);
+        return rc;
+    };
+    const int rc = mb->int8
+                       ? go(mb_beam_few_kernel<kPlanes, kF16, kNst, true>, (int)sizeof(MbFewSmem<kPlanes, true>) + 1024)
+                       : go(mb_beam_few_kernel<kPlanes, kF16, kNst, false>, (int)sizeof(MbFewSmem<kPlanes, false>) + 1024);
+    if (rc) return rc;
+    mb->last_pair = 0;
+    return check_launch("mb_beam_few_kernel");
+}
+
 template <int kPlanes, bool kF16, int kNst> int mb_launch_beam(vgb_multibeam *mb, const MbBeamArgs &a, cudaStream_t st)
 {
     const int v = g_mb_beam_variant.load();
     const bool pairs_ok = mb->mtiles % 2 == 0;
     if (v == 2 && !pairs_ok)
         return set_error(VGB_ERR_UNSUPPORTED, "multibeam: the pair kernel needs an even number of beam tiles");
+    if (mb->few) return mb_launch_beam_few<kPlanes, kF16, kNst>(mb, a, st);
     if (v == 0 && pairs_ok && mb->beam_pick == 0) {
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
@@ -1506,6 +1914,7 @@ extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibe
     mb->nint_p = (mb->nint + 127) / 128 * 128;
     mb->fp16 = c.precision == VGB_MB_FP16;
     mb->simt = c.precision == VGB_MB_FP32;
+    mb->few = !mb->simt && mb->mtiles == 1;
     mb->ntn = (c.nsamples + kMbUsed - 1) / kMbUsed;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -1526,7 +1935,9 @@ extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibe
     if (!rc && mb->simt) rc = mb_alloc(&mb->d_W32, nf * mb->Bp * 2 * A * 2, "FP32 weights");
     if (!rc && mb->simt) rc = mb_alloc(&mb->d_Q32, nf * mb->Mq * mb->KA, "FP32 autocorrelation weights");
     if (!rc && mb->simt) rc = check_cuda(cudaMemset(mb->d_Q32, 0, nf * mb->Mq * mb->KA * sizeof(float)), "cudaMemset");
-    if (!rc) rc = mb_alloc(&mb->d_V, nf * c.nsamples * mb->KA, "voltages");
+    // 16-bit operand rows, or the gathered input bytes (4 or 2 a tile and sample)
+    const size_t vrow = mb->few ? A * (mb->int8 ? 2 : 1) : (size_t)mb->KA;
+    if (!rc) rc = mb_alloc(&mb->d_V, nf * c.nsamples * vrow, "voltages");
     if (!rc) rc = mb_alloc(&mb->d_Aq, nf * mb->Mq * mb->Kq, "autocorrelation weights");
     if (!rc) rc = mb_alloc(&mb->d_C, nf * mb->nint_p * mb->Kb, "coherencies");
     if (!rc) rc = mb_alloc(&mb->d_qscale, nf * mb->Mq, "row scales");
@@ -1535,16 +1946,21 @@ extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibe
     if (!rc) rc = mb_alloc(&mb->d_stats, 3 * nf * c.npointing * c.nstokes, "row statistics");
     if (!rc)
         rc = check_cuda(cudaMemset(mb->d_Aq, 0, nf * mb->Mq * mb->Kq * sizeof(__half)), "cudaMemset");
+    if (!rc && mb->d_Aw && mb->Bp > c.npointing) // the padding beams' rows
+        rc = check_cuda(cudaMemset(mb->d_Aw, 0, mb->planes * nf * mb->Mrows * mb->KA * sizeof(uint16_t)), "cudaMemset");
     if (!rc) rc = check_cuda(cudaMemset(mb->d_C, 0, nf * mb->nint_p * mb->Kb * sizeof(__half)), "cudaMemset");
     if (!rc && !mb->simt)
         rc = make_tmap_bf16(&mb->tmW, mb->d_Aw, (uint64_t)mb->planes * nf * mb->Mrows, mb->KA, (uint64_t)mb->KA * 2,
                             128, mb->fp16);
-    if (!rc)
+    if (!rc && mb->few) {
+        rc = make_tmap_bytes(&mb->tmV, mb->d_V, (uint64_t)nf * c.nsamples, 2 * vrow, mb->int8 ? 64 : 32, kMbN);
+    } else if (!rc) {
         rc = make_tmap_bf16(&mb->tmV, mb->d_V, (uint64_t)nf * c.nsamples, mb->KA, (uint64_t)mb->KA * 2, kMbN,
                             mb->fp16);
-    if (!rc)
-        rc = make_tmap_bf16(&mb->tmV2, mb->d_V, (uint64_t)nf * c.nsamples, mb->KA, (uint64_t)mb->KA * 2, kMbN / 2,
-                            mb->fp16);
+        if (!rc)
+            rc = make_tmap_bf16(&mb->tmV2, mb->d_V, (uint64_t)nf * c.nsamples, mb->KA, (uint64_t)mb->KA * 2, kMbN / 2,
+                                mb->fp16);
+    }
     if (rc) {
         mb_free(mb);
         delete mb;
@@ -1657,10 +2073,15 @@ int mb_run_cc(vgb_multibeam *mb, int cc, const uint8_t *v_cc, float *S_cc, uint8
     w.stats = stats;
     w.B = c.npointing;
     if (A <= kMbPairMaxTiles && !mb->d_W32) {
+        // several beams a block share the channel's D^-1, as long as the blocks still fill the
+        // SMs (64 registers a thread): 20 beams of 128 tiles 35 us with 8 a block, 18 with 1
         const int threads = std::max(32, (A / 2 + 31) / 32 * 32);
-        mb_weights_pair_kernel<<<dim3((mb->Bp + kMbWeightBeams - 1) / kMbWeightBeams, nf), threads, 0, st>>>(w);
+        const long long fill = (long long)mb->nsm * (1024 / threads);
+        w.per_block = (int)std::min<long long>(kMbWeightBeams, std::max<long long>(1, (long long)c.npointing * nf / fill));
+        mb_weights_pair_kernel<<<dim3((c.npointing + w.per_block - 1) / w.per_block, nf), threads, 0, st>>>(w);
     } else {
-        mb_weights_kernel<<<dim3(mb->Bp, nf), kMbWeightThreads, 0, st>>>(w);
+        // (the FP32 mode's GEMM reads the padding beams' weights, the tensor kernels' stay zero)
+        mb_weights_kernel<<<dim3(mb->d_W32 ? mb->Bp : c.npointing, nf), kMbWeightThreads, 0, st>>>(w);
     }
     if ((rc = check_launch("mb_weights_kernel"))) return rc;
     mark(cc, 1);
@@ -1682,11 +2103,12 @@ int mb_run_cc(vgb_multibeam *mb, int cc, const uint8_t *v_cc, float *S_cc, uint8
     g.V = mb->d_V;
     g.C = mb->d_C;
     const int conv_smem = kMbInt * 2 * A * (mb->int8 ? 2 : 1);
-    if ((rc = check_cuda(cudaFuncSetAttribute(mb_convert_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              conv_smem),
+    auto conv = !mb->few ? mb_convert_kernel : mb->int8 ? mb_gather_voltages_kernel<true> : mb_gather_voltages_kernel<false>;
+    const int conv_threads = mb->few && !mb->int8 && A <= 128 ? 64 : 128;
+    if ((rc = check_cuda(cudaFuncSetAttribute(conv, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem),
                          "cudaFuncSetAttribute(mb_convert_kernel)")))
         return rc;
-    mb_convert_kernel<<<dim3(nf, mb->nint), 128, conv_smem, st>>>(g);
+    conv<<<dim3(nf, mb->nint), conv_threads, conv_smem, st>>>(g);
     if ((rc = check_launch("mb_convert_kernel"))) return rc;
     mark(cc, 2);
 
@@ -1779,7 +2201,11 @@ int mb_run_cc(vgb_multibeam *mb, int cc, const uint8_t *v_cc, float *S_cc, uint8
         r.out_st = out_st;
         r.offsets = off_cc;
         r.scales = scl_cc;
-        mb_renorm_kernel<<<dim3((nf + 31) / 32, c.npointing * c.nstokes), 256, 0, st>>>(r);
+        const dim3 rows((nf + 31) / 32, c.npointing * c.nstokes);
+        const long long shares = 16LL * mb->nsm / ((long long)rows.x * rows.y);
+        const int chunks = (mb->nint + kRnT - 1) / kRnT;
+        mb_renorm_kernel<<<dim3(rows.x, rows.y, (unsigned)std::min<long long>(chunks, std::max<long long>(1, shares))), 256, 0,
+                           st>>>(r);
         rc = check_launch("mb_renorm_kernel");
     }
     mark(cc, 5);

@@ -69,6 +69,25 @@ int make_tmap_bf16(CUtensorMap *map, const void *base, uint64_t rows, uint64_t c
     return VGB_SUCCESS;
 }
 
+int make_tmap_bytes(CUtensorMap *map, const void *base, uint64_t rows, uint64_t row_bytes, uint32_t box_bytes,
+                    uint32_t box_rows)
+{
+    auto fn = encode_fn();
+    if (!fn) return set_error(VGB_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+    if ((reinterpret_cast<uintptr_t>(base) & 15) || (row_bytes & 15) || (box_bytes & 15) || box_bytes == 0 ||
+        box_bytes > 256 || box_rows == 0 || box_rows > 256)
+        return set_error(VGB_ERR_INVALID, "tensor map: base, stride and box must be multiples of 16 bytes");
+    cuuint64_t dims[2] = {row_bytes, rows};
+    cuuint64_t strides[1] = {row_bytes};
+    cuuint32_t box[2] = {box_bytes, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void *>(base), dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error(VGB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    return VGB_SUCCESS;
+}
+
 int make_tmap_beam_weights(CUtensorMap *map, const void *W, int nant, int ncc, long long W_cc, int tiles_per_box)
 {
     auto fn = encode_fn();
