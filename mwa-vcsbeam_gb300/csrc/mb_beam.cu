@@ -231,10 +231,6 @@ __device__ __forceinline__ uint16_t to_bits(float x, bool fp16)
 {
     return fp16 ? __half_as_ushort(__float2half_rn(x)) : __bfloat16_as_ushort(__float2bfloat16_rn(x));
 }
-__device__ __forceinline__ float from_bits(uint16_t b, bool fp16)
-{
-    return fp16 ? __half2float(__ushort_as_half(b)) : __bfloat162float(__ushort_as_bfloat16(b));
-}
 
 // One block per (beam, channel); the threads step over tiles. Pass 1 finds the
 // largest |Q| of each Stokes row (its power-of-two scale), pass 2 writes the
@@ -254,6 +250,37 @@ __device__ __forceinline__ float2 mb_phase(const MbWeightArgs &w, int p, int a, 
     return make_float2(cs, sn);
 }
 
+// Four values -> 16-bit hi parts and the 16-bit remainders, two to a conversion
+// (1024 beams of 256 tiles: one at a time 1045 us, in pairs 977).
+__device__ __forceinline__ void mb_halves_bf16(const float (&v)[4], uint2 &hi2, uint2 &lo2)
+{
+    uint32_t hi[2], lo[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+        hi[j] = *reinterpret_cast<const uint32_t *>(&h);
+        const __nv_bfloat162 l = __floats2bfloat162_rn(v[2 * j] - __uint_as_float(hi[j] << 16),
+                                                       v[2 * j + 1] - __uint_as_float(hi[j] & 0xFFFF0000u));
+        lo[j] = *reinterpret_cast<const uint32_t *>(&l);
+    }
+    hi2 = make_uint2(hi[0], hi[1]);
+    lo2 = make_uint2(lo[0], lo[1]);
+}
+__device__ __forceinline__ void mb_halves_f16(const float (&v)[4], uint2 &hi2, uint2 &lo2)
+{
+    uint32_t hi[2], lo[2];
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const __half2 h = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+        hi[j] = *reinterpret_cast<const uint32_t *>(&h);
+        const float2 f = __half22float2(h);
+        const __half2 l = __floats2half2_rn(v[2 * j] - f.x, v[2 * j + 1] - f.y);
+        lo[j] = *reinterpret_cast<const uint32_t *>(&l);
+    }
+    hi2 = make_uint2(hi[0], hi[1]);
+    lo2 = make_uint2(lo[0], lo[1]);
+}
+
 // The embedded real rows (x, rho) of W = phase J^-1: four values per tile,
 // split into a hi part and the remainder (lo) in the GEMM's 16-bit type.
 __device__ __forceinline__ void mb_weight_halves(const float2 ph, const float2 (&J)[4], int x, int rho, bool h16,
@@ -265,27 +292,16 @@ __device__ __forceinline__ void mb_weight_halves(const float2 ph, const float2 (
         val[2 * q + 0] = rho == 0 ? v.x : v.y;
         val[2 * q + 1] = rho == 0 ? -v.y : v.x;
     }
-    uint16_t hi[4], lo[4];
-    for (int j = 0; j < 4; j++) {
-        hi[j] = to_bits(val[j], h16);
-        lo[j] = to_bits(val[j] - from_bits(hi[j], h16), h16);
-    }
-    hi2 = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
-    lo2 = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
+    if (h16) mb_halves_f16(val, hi2, lo2);
+    else mb_halves_bf16(val, hi2, lo2);
 }
 
 // Q row values scaled by inv_scale, split into FP16 hi and lo.
 __device__ __forceinline__ void mb_q_halves(const float (&q)[4], float inv_scale, uint2 &hi2, uint2 &lo2)
 {
-    uint16_t hi[4], lo[4];
-    for (int j = 0; j < 4; j++) {
-        const float s = q[j] * inv_scale;
-        const __half h = __float2half_rn(s);
-        hi[j] = __half_as_ushort(h);
-        lo[j] = __half_as_ushort(__float2half_rn(s - __half2float(h)));
-    }
-    hi2 = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
-    lo2 = make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
+    float s[4];
+    for (int j = 0; j < 4; j++) s[j] = q[j] * inv_scale;
+    mb_halves_f16(s, hi2, lo2);
 }
 
 // Power-of-two scale of each Stokes row of Q from the block's per-warp maxima.
