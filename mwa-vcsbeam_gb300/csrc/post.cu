@@ -799,7 +799,7 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 2) legacy4_kern
                 }
             }
         }
-        if (a.incoh) {
+        if (a.incoh && blockIdx.z == 0) {
 #pragma unroll
             for (int s = 0; s < kS; s++) {
                 for (int o = 4; o < 32; o <<= 1) power[s] += __shfl_xor_sync(0xffffffffu, power[s], o);
@@ -812,7 +812,7 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 2) legacy4_kern
     const int c = c0 + lane, part = warp % kParts;
     const bool live = c < a.nchan;
     const Word *vg = vt + (size_t)(warp / kParts) * ni * kL4C;
-    for (int p = 0; p < a.npointing; p++) {
+    for (int p = blockIdx.z; p < a.npointing; p += gridDim.z) {
         float2 acc[kS / 2][8];
 #pragma unroll
         for (int k = 0; k < kS / 2; k++)
@@ -919,26 +919,50 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kern
         const double2 *v = static_cast<const double2 *>(a.v) + ((long long)s0 * a.nchan + c0 + warp) * ni;
         const long long sstep = (long long)a.nchan * ni;
         const int ns = min(kS * kG, a.nsamples - s0);
-        // short rows: 32 / ni of them side by side in the warp
-        const int side = ni < 32 ? 32 / ni : 1, sub = ni < 32 ? lane / ni : 0, i0 = ni < 32 ? lane % ni : lane;
-        constexpr int kFly = kPairs * kG >= 2 ? 2 : 1;
-        for (int k0 = sub; k0 < kPairs * kG && sub < side; k0 += kFly * side)
+        constexpr int kRows = kPairs * kG;
+        if (((ni + 31) & ~31) * 8 <= ni * 9) {
+            constexpr int kFly = kRows >= 2 ? 2 : 1;
+            for (int k0 = 0; k0 < kRows; k0 += kFly)
 #pragma unroll 2
-            for (int i = i0; i < ni; i += 32) {
+                for (int i = lane; i < ni; i += 32) {
+                    double2 d[kFly][2];
+#pragma unroll
+                    for (int k = 0; k < kFly; k++)
+#pragma unroll
+                        for (int q = 0; q < 2; q++) {
+                            const int sl = 2 * (k0 + k) + q;
+                            d[k][q] = sl < ns ? __ldcs(v + sl * sstep + i) : make_double2(0.0, 0.0);
+                        }
+#pragma unroll
+                    for (int k = 0; k < kFly; k++)
+                        vt[((k0 + k) * kLdC + warp) * stride + i] = narrow4(d[k][0].x, d[k][1].x, d[k][0].y, d[k][1].y);
+                }
+        } else {
+            // more than an eighth of the lanes would idle at the rows' ends: the rows as one run over
+            // the lanes (20 tiles, 3,000 samples, one beam: 95 -> 60 us; whole rows of 128 tiles the
+            // other way, 283 -> 311 us for the work around it)
+            constexpr int kFly = 4;
+            const int dk = 32 / ni, di = 32 - dk * ni;
+            int k = lane / ni, i = lane - k * ni;
+            while (k < kRows) {
                 double2 d[kFly][2];
+                int at[kFly];
 #pragma unroll
-                for (int k = 0; k < kFly; k++)
+                for (int f = 0; f < kFly; f++) {
+                    at[f] = k < kRows ? (k * kLdC + warp) * stride + i : -1;
 #pragma unroll
-                    for (int q = 0; q < 2; q++) {
-                        const int sl = 2 * (k0 + k * side) + q;
-                        d[k][q] = sl < ns ? __ldcs(v + sl * sstep + i) : make_double2(0.0, 0.0);
-                    }
+                    for (int q = 0; q < 2; q++)
+                        d[f][q] = 2 * k + q < ns ? __ldcs(v + (2 * k + q) * sstep + i) : make_double2(0.0, 0.0);
+                    i += di;
+                    const int next = i >= ni;
+                    i -= next ? ni : 0;
+                    k += dk + next;
+                }
 #pragma unroll
-                for (int k = 0; k < kFly; k++)
-                    if (k0 + k * side < kPairs * kG)
-                        vt[((k0 + k * side) * kLdC + warp) * stride + i] =
-                            narrow4(d[k][0].x, d[k][1].x, d[k][0].y, d[k][1].y);
+                for (int f = 0; f < kFly; f++)
+                    if (at[f] >= 0) vt[at[f]] = narrow4(d[f][0].x, d[f][1].x, d[f][0].y, d[f][1].y);
             }
+        }
     }
     __syncthreads();
 
@@ -946,7 +970,7 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kern
     const int part = 4 * (warp % kGroupWarps) + (lane >> 3);
     const bool live = c < a.nchan;
     const float4 *vc = vt + (group * kPairs * kLdC + cl) * stride;
-    for (int p = 0; p < a.npointing; p++) {
+    for (int p = blockIdx.z; p < a.npointing; p += gridDim.z) {
         float2 acc[kPairs][8];
 #pragma unroll
         for (int k = 0; k < kPairs; k++)
@@ -1012,23 +1036,25 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kern
 }
 
 // The tile: as many sample groups as leave two (4-bit) or three (FP64) blocks'
-// shared memory per SM, so that small arrays spend less on the partial sums
-// (8 tiles of FP64 voltages, 1,000 samples: 29 us with one group, 15 us with
-// eight, 17 us with the row kernel); where one group of the larger kS leaves
-// room for one block only, the smaller kS (256 tiles of 4+4-bit voltages, 4,000
-// samples: 224 us, row kernel 840 us). Arrays past that (more than 768 tiles of
-// 4+4-bit or 877 of FP64 voltages) take the row kernel.
+// shared memory per SM and still give every SM a block (4-bit, pointings counted:
+// they can go to different blocks) or two (FP64): groups spend less on the partial
+// sums, but a short run needs its samples spread (4-bit, 8 tiles, 200 samples, one
+// beam: 10.9 us in 16-sample tiles, 8.8 in 8; 3,000 samples: 21.2 and 24.2; FP64,
+// 8 tiles, one beam, 3,000 samples: 31 us with eight groups, 70 with one). The row
+// kernel takes 8.8 and 35.5 us for the 4-bit runs, 40 us for the FP64 one. Where
+// one group of the larger kS leaves room for one block only, the smaller kS (256
+// tiles of 4+4-bit voltages, 4,000 samples: 224 us, row kernel 840 us). Arrays past
+// that (more than 768 tiles of 4+4-bit or 877 of FP64 voltages) take the row kernel.
 struct LegacyTile {
     void (*kern)(LegacyArgs);
     size_t smem;
     int channels, samples;
 };
 
-static LegacyTile legacy_tile(bool int4, int nant)
+static LegacyTile legacy_tile(const LegacyArgs &a, bool int4, int nsm)
 {
-    const LegacyTile t4[] = {{legacy4_kernel<8, 8>, legacy4_smem<8, 8>(nant), kL4C, 64},
-                             {legacy4_kernel<8, 4>, legacy4_smem<8, 4>(nant), kL4C, 32},
-                             {legacy4_kernel<8, 2>, legacy4_smem<8, 2>(nant), kL4C, 16},
+    const int nant = a.nant;
+    const LegacyTile t4[] = {{legacy4_kernel<8, 2>, legacy4_smem<8, 2>(nant), kL4C, 16},
                              {legacy4_kernel<8, 1>, legacy4_smem<8, 1>(nant), kL4C, 8},
                              {legacy4_kernel<4, 1>, legacy4_smem<4, 1>(nant), kL4C, 4}};
     const LegacyTile td[] = {{legacyd_kernel<4, 8>, legacyd_smem<4, 8>(nant), kLdC, 32},
@@ -1037,9 +1063,14 @@ static LegacyTile legacy_tile(bool int4, int nant)
                              {legacyd_kernel<4, 1>, legacyd_smem<4, 1>(nant), kLdC, 4},
                              {legacyd_kernel<2, 1>, legacyd_smem<2, 1>(nant), kLdC, 2}};
     const LegacyTile *t = int4 ? t4 : td;
-    for (int k = 0; k < 4; k++)
-        if (t[k].smem <= (size_t)(int4 ? 113 : k < 3 ? 75 : 113) * 1024) return t[k];
-    return t[4];
+    const int n = int4 ? 3 : 5;
+    for (int k = 0; k < n - 1; k++) {
+        const long long blocks = (long long)((a.nchan + t[k].channels - 1) / t[k].channels) *
+                                 ((a.nsamples + t[k].samples - 1) / t[k].samples);
+        const bool enough = k == n - 2 || (int4 ? blocks * a.npointing >= nsm : blocks >= 2 * nsm);
+        if (enough && t[k].smem <= (size_t)(int4 || k == n - 2 ? 113 : 75) * 1024) return t[k];
+    }
+    return t[n - 1];
 }
 
 // ---------------------------------------------------------------------------
@@ -1172,12 +1203,20 @@ int launch_legacy_beam(const LegacyArgs &a, cudaStream_t st)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: %d inputs do not fit the shared-memory tile", ni);
     if ((a.nsamples + kLS - 1) / kLS > 65535)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: at most %d samples per call", 65535 * kLS);
-    const LegacyTile t = legacy_tile(int4, a.nant);
+    int nsm = 1, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return check_cuda(cudaGetLastError(), "cudaDeviceGetAttribute(legacy)");
+    const LegacyTile t = legacy_tile(a, int4, nsm);
     if (t.smem <= 227 * 1024) {
         const int rc = check_cuda(cudaFuncSetAttribute(t.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem),
                                   "cudaFuncSetAttribute(legacy tile)");
         if (rc) return rc;
-        t.kern<<<dim3((a.nchan + t.channels - 1) / t.channels, (a.nsamples + t.samples - 1) / t.samples), 256, t.smem, st>>>(a);
+        const unsigned gx = (a.nchan + t.channels - 1) / t.channels, gy = (a.nsamples + t.samples - 1) / t.samples;
+        // the pointings over blocks too where the rest is short of two (4-bit) or one (FP64) per SM: each
+        // share reads the voltages again (4-bit, 20 tiles, 200 samples, 12 beams: 74 -> 21 us)
+        const long long shares = (int4 ? 2 : 1) * nsm / ((long long)gx * gy);
+        const unsigned gz = (unsigned)std::min<long long>(a.npointing, std::max<long long>(1, shares));
+        t.kern<<<dim3(gx, gy, gz), 256, t.smem, st>>>(a);
         return check_launch("legacy beam kernel");
     }
     dim3 grid((a.nchan + kLC - 1) / kLC, (a.nsamples + kLS - 1) / kLS);

@@ -48,6 +48,10 @@ CASES = [  # double, tiles, channels, samples, pointings, Stokes
     (True, 1, 1, 1, 1, 1), (True, 5, 9, 33, 2, 4), (True, 17, 7, 31, 1, 4), (True, 33, 16, 17, 3, 1),
     (True, 65, 9, 9, 1, 4), (True, 128, 9, 5, 2, 4), (True, 145, 8, 3, 1, 4), (True, 255, 3, 5, 2, 4),
     (True, 890, 2, 3, 1, 4),
+    # enough blocks for several sample groups a block, with a partial last group; pointings over the blocks
+    (False, 6, 128, 619, 1, 4), (False, 36, 120, 333, 2, 4), (False, 8, 128, 21, 5, 4), (False, 130, 64, 9, 7, 1),
+    (True, 5, 127, 615, 1, 4), (True, 20, 128, 307, 2, 4), (True, 33, 128, 157, 1, 1), (True, 128, 128, 78, 2, 4),
+    (True, 21, 64, 11, 6, 4),
 ]
 
 
