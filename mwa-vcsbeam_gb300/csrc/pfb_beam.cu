@@ -1460,12 +1460,16 @@ template <int A, bool B, bool C> struct BeamSel {
 template <int A, bool B, bool C> struct PackSel {
     static int run(const PackArgs &a, dim3 grid, cudaStream_t st)
     {
-        constexpr size_t base = sizeof(PackSmem);
+        // Complex-double rows: two CTAs per SM (by the shared memory asked for). Every CTA has
+        // 1,024 rows open, a 64-byte run of each per step; with three per SM the lines waiting for
+        // their other half outgrow L2 and go out in pieces (3 channels, 3,901 spectra, FP32 sums:
+        // 117 tiles 2,023 -> 1,584 us, 128 tiles 1,692 -> 1,553). The 4-bit rows stay at three.
+        constexpr size_t base = sizeof(PackSmem), least = C ? 0 : 80 * 1024;
         int rc = check_cuda(cudaFuncSetAttribute(pack_kernel<A, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)(base + sizeof(int) * kPackMaxInputs)),
+                                                 (int)std::max(least, base + sizeof(int) * kPackMaxInputs)),
                             "cudaFuncSetAttribute(pack smem)");
         if (rc) return rc;
-        const size_t smem = base + sizeof(int) * (size_t)a.vv.ninputs;
+        const size_t smem = std::max(least, base + sizeof(int) * (size_t)a.vv.ninputs);
         // Each CTA takes a share of the steps (the columns are independent), a
         // multiple of 4 (16 columns: the 4-bit mode's wide stores), so that the
         // last wave is a small part: about 12 waves of CTAs, at least 8 steps
