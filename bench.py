@@ -628,8 +628,8 @@ def gb300_arm(args, rank, local_rank, world):
     if variant == 5:
         kname = "beam_tm_kernel (fused PFB + tied-array/incoherent beam + Stokes; three CTAs per SM)"
         limiter = ("not HBM: the FMA pipe and the shared-memory pipe, each ~60 % busy (ncu of a 2-channel "
-                   "launch: issue 62.7 %, FMA pipe 56.0 %, shared-memory wavefronts 63 % of peak, conversions "
-                   "on the XU pipe 17.3 %, math-pipe throttle the second stall reason; DRAM 1.41 GB in 1.854 ms)")
+                   "launch: issue 64.3 %, FMA pipe 56.5 %, shared-memory pipe 55 % of peak, math-pipe "
+                   "throttle the second stall reason; 1.789 ms)")
     else:
         kname = "beam_kernel (fused PFB + tied-array/incoherent beam + Stokes)"
         limiter = ("not HBM: instruction issue, the FMA pipe and the shared-memory pipe, each ~60 % busy "

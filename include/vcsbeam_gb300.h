@@ -337,7 +337,7 @@ int vgb_vdif_advance(uint32_t *d_hdr, int njobs, int nframes, void *stream);
  * the GPU's memory and before any stream capture. A call with nspectra = 0
  * does only that set-up (its other pointers may be NULL). Setting
  * CUDA_MODULE_LOADING=EAGER places the array when the library loads instead.
- * The first call for each new shape also times the fused front end's two
+ * The first call for each new shape also times the fused front end's three
  * tile shapes once (extra launches and a wait on CUDA events, see
  * vgb_pfb_variant); force one with vgb_pfb_variant(4) to skip that.
  * All calls share the one array, which keeps the last call's contents.
@@ -565,8 +565,9 @@ int vgb_multibeam_launches(const vgb_multibeam *mb);
  * half of the voltage tile) against the single-CTA kernel on its first coarse
  * channel, two launches each, waits for them, and keeps the faster (a first
  * run inside a capture takes the pair kernel); otherwise the single-CTA
- * kernel. 1 the single-CTA kernel; 2 the pair kernel or an error. Returns the
- * previous setting (-1 on a bad value). */
+ * kernel. 1 the single-CTA kernel; 2 the pair kernel or an error. Up to 32
+ * beams (one tile) run a single-CTA kernel of their own, whose voltages stay
+ * input bytes in memory. Returns the previous setting (-1 on a bad value). */
 int vgb_multibeam_beam_variant(int v);
 /* CTA pairs (2-CTA clusters) the last beam GEMM ran on; 0 if it ran the
  * single-CTA kernel. */
