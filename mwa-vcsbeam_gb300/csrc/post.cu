@@ -495,10 +495,12 @@ template <int kCh, bool kStats> __global__ void __launch_bounds__(256, 5) renorm
             }
             if (isnan(s0)) lo = hi = s0;
         }
-        // no block leaves while another still reads its partials: arrive now
-        // (the reads are done, nothing is published), wait at the end
+        // no block leaves while another still reads its partials: arrive now, wait
+        // at the end. The arrival is a release: a relaxed one would order none of
+        // the remote reads before it, and a block without samples could be gone
+        // while they are in flight
         __syncwarp();
-        asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     }
     if (tid < kCh) {
         const float scale = (float)((double)(hi - lo) / 256.0);
@@ -530,7 +532,7 @@ template <int kCh, bool kStats> __global__ void __launch_bounds__(256, 5) renorm
 #pragma unroll 2
         for (int s = sb + row; s < se; s += kRows) put(s, rsm[(s - sb) * kQ + q]);
         __syncwarp();
-        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 }
 
