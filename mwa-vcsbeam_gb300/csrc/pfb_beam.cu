@@ -767,6 +767,7 @@ __device__ __forceinline__ void beam_tm_body(const BeamArgs &a, const CUtensorMa
         mbar_init(&sm.bar_w, 1);
         fence_mbar_init();
     }
+    __syncwarp(); // allocation and accesses of tensor memory are warp-collective, and lane 0 was alone
     if (warp == 0) {
         tmem_alloc(&sm.tmem, kTmCols);
         tmem_relinquish();
@@ -781,6 +782,7 @@ __device__ __forceinline__ void beam_tm_body(const BeamArgs &a, const CUtensorMa
         tm_frames<T>(sm, a.vv, cc, 0, m0, a.nspectra, a.status);
         tm_weights(sm, wmap, cc, 0);
     }
+    __syncwarp(); // lane 0 has copied
     if (warp < 4) tm_tables<kW, kFpga>(ttab, a.filter, tid);
     tc_fence_before();
     __syncthreads();
@@ -795,6 +797,7 @@ __device__ __forceinline__ void beam_tm_body(const BeamArgs &a, const CUtensorMa
         if (__syncthreads_or(!got || wbad)) break;
         if (it > 0) tm_weights(sm, wmap, cc, it);
         if (kStages == 2 && it + 1 < nsteps) tm_frames<T>(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
+        __syncwarp(); // lane 0 has copied
         {
             typename WolaTap<kW>::type t[kP];
             tm_taps<kW>(ttab, t);
@@ -1186,6 +1189,7 @@ __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kerne
     tc_fence_after();
     const uint32_t tlane = sm.tmem + ((uint32_t)(32 * ((tid >> 5) & 3)) << 16), ttab = tlane + kPackTables;
     pack_frames(sm, a.vv, cc, step0, m0, a.nspectra, a.status, inv);
+    __syncwarp(); // the tensor-memory accesses are warp-collective, and lane 0 has copied
     if (tid < 128) tm_tables<kW, kFpga>(ttab, a.filter, tid);
     tc_fence_before();
     __syncthreads();
