@@ -1888,6 +1888,28 @@ template <int kPlanes, bool kF16, int kNst> int mb_launch_beam(vgb_multibeam *mb
     return mb_launch_beam_single<kPlanes, kF16, kNst>(mb, a, st);
 }
 
+// The rows and columns of padding, zeroed once. Runs come on any stream, ordered
+// behind nothing that happens here, so this has completed when it returns; on a
+// stream of its own, so that it neither waits for nor holds up other work.
+int mb_zero(vgb_multibeam *mb)
+{
+    const size_t nf = mb->cfg.nfine;
+    cudaStream_t st;
+    int rc = check_cuda(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+    if (rc) return rc;
+    auto zero = [&](void *p, size_t bytes) {
+        if (!rc) rc = check_cuda(cudaMemsetAsync(p, 0, bytes, st), "cudaMemsetAsync");
+    };
+    if (mb->d_Q32) zero(mb->d_Q32, nf * mb->Mq * mb->KA * sizeof(float));
+    zero(mb->d_Aq, nf * mb->Mq * mb->Kq * sizeof(__half));
+    if (mb->d_Aw && mb->Bp > mb->cfg.npointing) // the padding beams' rows
+        zero(mb->d_Aw, mb->planes * nf * mb->Mrows * mb->KA * sizeof(uint16_t));
+    zero(mb->d_C, nf * mb->nint_p * mb->Kb * sizeof(__half));
+    const int done = check_cuda(cudaStreamSynchronize(st), "cudaStreamSynchronize");
+    cudaStreamDestroy(st);
+    return rc ? rc : done;
+}
+
 } // namespace
 
 extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibeam **out)
@@ -1950,7 +1972,6 @@ extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibe
     if (!rc && !mb->simt) rc = mb_alloc(&mb->d_Aw, (size_t)mb->planes * nf * mb->Mrows * mb->KA, "weights");
     if (!rc && mb->simt) rc = mb_alloc(&mb->d_W32, nf * mb->Bp * 2 * A * 2, "FP32 weights");
     if (!rc && mb->simt) rc = mb_alloc(&mb->d_Q32, nf * mb->Mq * mb->KA, "FP32 autocorrelation weights");
-    if (!rc && mb->simt) rc = check_cuda(cudaMemset(mb->d_Q32, 0, nf * mb->Mq * mb->KA * sizeof(float)), "cudaMemset");
     // 16-bit operand rows, or the gathered input bytes (4 or 2 a tile and sample)
     const size_t vrow = mb->few ? A * (mb->int8 ? 2 : 1) : (size_t)mb->KA;
     if (!rc) rc = mb_alloc(&mb->d_V, nf * c.nsamples * vrow, "voltages");
@@ -1960,11 +1981,7 @@ extern "C" int vgb_multibeam_create(const vgb_multibeam_config *cfg, vgb_multibe
     if (!rc) rc = mb_alloc(&mb->d_R, nf * mb->Mq * mb->nint_p, "autocorrelation terms");
     if (!rc) rc = mb_alloc(&mb->d_S, nf * c.npointing * c.nstokes * mb->nint, "Stokes");
     if (!rc) rc = mb_alloc(&mb->d_stats, 3 * nf * c.npointing * c.nstokes, "row statistics");
-    if (!rc)
-        rc = check_cuda(cudaMemset(mb->d_Aq, 0, nf * mb->Mq * mb->Kq * sizeof(__half)), "cudaMemset");
-    if (!rc && mb->d_Aw && mb->Bp > c.npointing) // the padding beams' rows
-        rc = check_cuda(cudaMemset(mb->d_Aw, 0, mb->planes * nf * mb->Mrows * mb->KA * sizeof(uint16_t)), "cudaMemset");
-    if (!rc) rc = check_cuda(cudaMemset(mb->d_C, 0, nf * mb->nint_p * mb->Kb * sizeof(__half)), "cudaMemset");
+    if (!rc) rc = mb_zero(mb);
     if (!rc && !mb->simt)
         rc = make_tmap_bf16(&mb->tmW, mb->d_Aw, (uint64_t)mb->planes * nf * mb->Mrows, mb->KA, (uint64_t)mb->KA * 2,
                             128, mb->fp16);
