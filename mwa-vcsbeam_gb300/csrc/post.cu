@@ -11,6 +11,7 @@
 //    (v_IDX [s][c][i], 4+4-bit or complex FP64): vmApplyJ_kernel followed by
 //    vmBeamform_kernel (form_beam.cpp:122-371) in one pass.
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include <cooperative_groups.h>
@@ -699,6 +700,15 @@ __device__ __forceinline__ void legacy_store(const LegacyArgs &a, int p, int s, 
     if (a.e) a.e[((long long)p * a.nsamples + s) * a.nchan + c] = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
+// Tiles of channels and samples on grid x, channels fastest: two samples a tile
+// make more sample tiles than grid y counts (65,535) well within a call's limit.
+template <int kCh, int kSamp> __device__ __forceinline__ void legacy_origin(const LegacyArgs &a, int &c0, int &s0)
+{
+    const unsigned across = (unsigned)(a.nchan + kCh - 1) / kCh;
+    c0 = (int)(blockIdx.x % across) * kCh;
+    s0 = (int)(blockIdx.x / across) * kSamp;
+}
+
 // The tiles' (Q, P) input pairs into shared memory, checked against the row.
 __device__ __forceinline__ void legacy_inputs(const LegacyArgs &a, uint32_t *pq)
 {
@@ -706,7 +716,7 @@ __device__ __forceinline__ void legacy_inputs(const LegacyArgs &a, uint32_t *pq)
     for (int ant = threadIdx.x; ant < a.nant; ant += blockDim.x) {
         uint32_t iq = __ldg(a.polQ + ant), ip = __ldg(a.polP + ant);
         if (iq >= ni || ip >= ni) {
-            if (blockIdx.x == 0 && blockIdx.y == 0) atomicOr(a.status, kErrBadInput);
+            if (blockIdx.x == 0) atomicOr(a.status, kErrBadInput);
             iq = ip = 0;
         }
         pq[ant] = iq | (ip << 16);
@@ -756,7 +766,8 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 2) legacy4_kern
     Word *vt = reinterpret_cast<Word *>(red + kL4Red);
     uint32_t *pq = reinterpret_cast<uint32_t *>(vt + (size_t)kG * ni * kL4C);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int c0 = blockIdx.x * kL4C, s0 = blockIdx.y * kS * kG;
+    int c0, s0;
+    legacy_origin<kL4C, kS * kG>(a, c0, s0);
 
     legacy_inputs(a, pq);
     // stage: lane = (channel 4 warp + lane % 4, word lane / 4 of 8), so 8 lanes
@@ -913,7 +924,8 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kern
     float *red = reinterpret_cast<float *>(vt + (size_t)kPairs * kG * kLdC * stride); // partial sums
     uint32_t *pq = reinterpret_cast<uint32_t *>(red + kLWarps * kS * 8 * kLdC);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int c0 = blockIdx.x * kLdC, s0 = blockIdx.y * kS * kG;
+    int c0, s0;
+    legacy_origin<kLdC, kS * kG>(a, c0, s0);
 
     legacy_inputs(a, pq);
     // warp w stages channel w's rows, two sample pairs in flight
@@ -1209,16 +1221,16 @@ int launch_legacy_beam(const LegacyArgs &a, cudaStream_t st)
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return check_cuda(cudaGetLastError(), "cudaDeviceGetAttribute(legacy)");
     const LegacyTile t = legacy_tile(a, int4, nsm);
-    if (t.smem <= 227 * 1024) {
+    const long long blocks = (long long)((a.nchan + t.channels - 1) / t.channels) * ((a.nsamples + t.samples - 1) / t.samples);
+    if (t.smem <= 227 * 1024 && blocks <= INT_MAX) {
         const int rc = check_cuda(cudaFuncSetAttribute(t.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem),
                                   "cudaFuncSetAttribute(legacy tile)");
         if (rc) return rc;
-        const unsigned gx = (a.nchan + t.channels - 1) / t.channels, gy = (a.nsamples + t.samples - 1) / t.samples;
         // the pointings over blocks too where the rest is short of two (4-bit) or one (FP64) per SM: each
         // share reads the voltages again (4-bit, 20 tiles, 200 samples, 12 beams: 74 -> 21 us)
-        const long long shares = (int4 ? 2 : 1) * nsm / ((long long)gx * gy);
+        const long long shares = (int4 ? 2 : 1) * nsm / blocks;
         const unsigned gz = (unsigned)std::min<long long>(a.npointing, std::max<long long>(1, shares));
-        t.kern<<<dim3(gx, gy, gz), 256, t.smem, st>>>(a);
+        t.kern<<<dim3((unsigned)blocks, 1, gz), 256, t.smem, st>>>(a);
         return check_launch("legacy beam kernel");
     }
     dim3 grid((a.nchan + kLC - 1) / kLC, (a.nsamples + kLS - 1) / kLS);
