@@ -26,6 +26,8 @@
 // of the reference's doc/Definitions.md): horizon (az, el) -> (ha, dec) at
 // latitude lat, chi = atan2(cos lat sin ha, sin lat cos dec - cos lat sin dec
 // cos ha), P = [[-cos chi, -sin chi], [sin chi, -cos chi]], B = J P.
+#include <algorithm>
+
 #include "beam_model.cuh"
 #include "vgb_launch.cuh"
 
@@ -59,117 +61,162 @@ __device__ __forceinline__ void bm_store(double2 *o, const double2 (&J)[4], cons
         }
 }
 
-// bm_jones by 16 lanes (l = 0 .. 15 of `mask`), one dipole each: the same
-// operations, the dipoles' terms added in dipole order. Every lane returns J.
-__device__ __forceinline__ void bm_jones16(int l, unsigned mask, double az, double za, double f, const uint32_t *d,
-                                           double2 (&J)[4])
+// What bm_jones computes once per direction and frequency: p holds bm_project's
+// projections in its order.
+struct BmDir {
+    double saz, caz, sza, k, g, p[4];
+};
+
+// By two lanes (l = 0, 1) of `mask`'s pairs, a sine each; both return it.
+__device__ __forceinline__ BmDir bm_dir2(int l, unsigned mask, double az, double za, double f)
 {
     double s, c;
     sincos(l == 0 ? az : za, &s, &c);
-    const double saz = __shfl_sync(mask, s, 0, 16), caz = __shfl_sync(mask, c, 0, 16);
-    const double sza = __shfl_sync(mask, s, 1, 16), cza = __shfl_sync(mask, c, 1, 16);
-    const double k = 2.0 * kBmPi * f;
-    const uint32_t di = d[l];
-    bm_dipole(l, di, sza, saz, caz, k, s, c);
-    double re = 0.0, im = 0.0;
-    int live = 0;
-    for (int i = 0; i < 16; i++) {
-        const double ci = __shfl_sync(mask, c, i, 16), si = __shfl_sync(mask, s, i, 16);
-        if (__shfl_sync(mask, di, i, 16) == 32u) continue;
-        live++;
-        re += ci;
-        im += si;
-    }
-    const double gl = sin(l == 0 ? k * kBmHeight * cza / kBmC : k * kBmHeight / kBmC);
-    bm_project(live, re, im, __shfl_sync(mask, gl, 0, 16) / __shfl_sync(mask, gl, 1, 16), saz, caz, cza, J);
+    BmDir v;
+    v.saz = __shfl_sync(mask, s, 0, 2), v.caz = __shfl_sync(mask, c, 0, 2);
+    v.sza = __shfl_sync(mask, s, 1, 2);
+    const double cza = __shfl_sync(mask, c, 1, 2);
+    v.k = 2.0 * kBmPi * f;
+    const double gl = sin(l == 0 ? v.k * kBmHeight * cza / kBmC : v.k * kBmHeight / kBmC);
+    v.g = __shfl_sync(mask, gl, 0, 2) / __shfl_sync(mask, gl, 1, 2);
+    v.p[0] = cza * v.saz, v.p[1] = cza * v.caz, v.p[2] = v.caz, v.p[3] = -v.saz;
+    return v;
 }
 
-// Everything in one launch: block b takes (frequency, pointing) pairs b *
-// per_block ... and writes their B for all tiles. A chain of FP64
-// transcendentals (about 2 us each at this GPU's FP64 latency) bounds a small
-// call, so a delay set's 16 dipoles take 16 lanes, the parallactic rotations
-// one lane each of the last warp beside them, and the tiles' sets are found in
-// shared memory by every block instead of a kernel of its own: 8 to 152
-// pointings x 128 tiles in 3 sets, 78-88 us in three launches -> 19 us. The
-// lanes repeat the per-direction work, 6.1 ns per (pair, set) against 4.3 ns
-// with one thread each, so past 304 pairs (24,576 pairs: 453 against 317 us) the
-// three launches take over.
+// bm_jones and bm_store by 16 lanes (l = 0 .. 15 of `mask`) with the same
+// operations: a dipole's phase term each, the terms added in dipole order (real
+// parts on even lanes, imaginary parts on odd ones), then lanes 0 .. 7 write one
+// of the matrix's eight values each.
+__device__ __forceinline__ void bm_write16(int l, unsigned mask, const BmDir &v, const uint32_t *d, const double *P,
+                                           double2 *o)
+{
+    const uint32_t di = d[l];
+    double s, c, sum = 0.0;
+    bm_dipole(l, di, v.sza, v.saz, v.caz, v.k, s, c);
+    const unsigned live = __ballot_sync(mask, di != 32u) >> (__ffs(mask) - 1);
+    for (int i = 0; i < 16; i++) {
+        const double ci = __shfl_sync(mask, c, i, 16), si = __shfl_sync(mask, s, i, 16);
+        if (live >> i & 1u) sum += l & 1 ? si : ci;
+    }
+    if (l >= 8) return;
+    const int r = l >> 2, col = l >> 1 & 1;
+    const double q = sum / 16.0 * v.g;
+    const double ja = live ? q * v.p[2 * r] : 0.0, jb = live ? q * v.p[2 * r + 1] : 0.0;
+    reinterpret_cast<double *>(o)[l] = P ? fma(jb, P[2 + col], __dmul_rn(ja, P[col])) : col ? jb : ja;
+}
+
+// Everything in one launch: block (b, y) takes (frequency, pointing) pairs b *
+// per_block ... and the distinct delay sets y, y + gridDim.y, ...; it writes B for
+// the tiles of those sets. A chain of FP64 transcendentals (about 2 us each at this
+// GPU's FP64 latency) bounds a small call, so a delay set's 16 dipoles take 16
+// lanes, and the directions and the parallactic rotations a warp each while the
+// others find the sets in shared memory, which every block does instead of a kernel
+// of its own. With many sets the FP64 pipe bounds it (2 per clock per SM): what
+// depends on the direction only is computed once per pair, no sum or product is
+// formed by two lanes, and the sets go to as many blocks as there are SMs (how many
+// sets there are is not known to the host, so blocks past them leave). With 3 / all
+// tiles different, against the three launches (us):
+//   8 pointings, 128 tiles    17 / 19    63 / 75     152, 128 tiles    17 / 51    68 / 77
+//   1 pointing, 2,048 tiles   44 / 109  145 / 382    304, 256 tiles    19 / 159   76 / 217
+// Measured up to 304 pairs; many more fill the GPU with a thread per (pair, set).
 constexpr int kBmThreads = 256, kBmPairs = 2, kBmMaxTiles = 2048, kBmMaxPairs = 304;
+constexpr int kBmFinders = kBmThreads - 64, kBmGroups = kBmThreads / 16;
+
+__host__ __device__ constexpr int bm_hashes(int ntile) { return (ntile + 15) / 16 * 16; }
+
+// The first tile with tile t's delays.
+__device__ __forceinline__ int bm_first_equal(const uint32_t *hash, const uint32_t *delays, int t)
+{
+    const uint32_t h = hash[t];
+    for (int u = 0; u < t; u += 16) {
+        bool any = false;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint4 q = reinterpret_cast<const uint4 *>(hash + u)[j];
+            any |= q.x == h || q.y == h || q.z == h || q.w == h;
+        }
+        if (any)
+            for (int w = u; w < min(u + 16, t); w++)
+                if (hash[w] == h && same_delays(delays, t, w)) return w;
+    }
+    return t;
+}
 
 __global__ void __launch_bounds__(kBmThreads) beam_kernel_fused(const PbArgs a, int per_block)
 {
-    extern __shared__ int bm_smem[];
-    int *rep = bm_smem, *list = rep + a.ntile;
-    uint32_t *hash = reinterpret_cast<uint32_t *>(list + a.ntile);
+    extern __shared__ __align__(16) int bm_smem[];
+    uint32_t *hash = reinterpret_cast<uint32_t *>(bm_smem);
+    int *rep = bm_smem + bm_hashes(a.ntile), *list = rep + a.ntile, *rank = list + a.ntile;
     __shared__ double P[kBmPairs][4];
-    __shared__ int warp_count[kBmThreads / 32];
+    __shared__ BmDir dir[kBmPairs];
+    __shared__ int warp_count[kBmFinders / 32], nlist;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long pairs = (long long)a.nfreq * a.npointing;
     const long long p0 = (long long)blockIdx.x * per_block;
     const int np = (int)min((long long)per_block, pairs - p0);
 
-    for (int t = tid; t < a.ntile; t += kBmThreads) {
-        uint32_t h = 2166136261u;
-        for (int i = 0; i < 16; i++) h = (h ^ a.delays[16 * (long long)t + i]) * 16777619u;
-        hash[t] = h;
+    if (tid < kBmFinders) {
+        for (int t = tid; t < a.ntile; t += kBmFinders) {
+            uint32_t h = 2166136261u;
+            for (int i = 0; i < 16; i++) h = (h ^ a.delays[16 * (long long)t + i]) * 16777619u;
+            hash[t] = h;
+        }
+        auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"(kBmFinders) : "memory"); };
+        meet();
+        // rep[t]: the first tile with tile t's delays; list: those first tiles; rank: their places in it
+        int count = 0;
+        for (int t0 = 0; t0 < a.ntile; t0 += kBmFinders) {
+            const int t = t0 + tid;
+            const int r = t < a.ntile ? bm_first_equal(hash, a.delays, t) : -1;
+            if (t < a.ntile) rep[t] = r;
+            const bool first = r == t;
+            __syncwarp();
+            const unsigned b = __ballot_sync(0xffffffffu, first);
+            if (lane == 0) warp_count[warp] = __popc(b);
+            meet();
+            int at = count;
+            for (int w = 0; w < kBmFinders / 32; w++) {
+                if (w < warp) at += warp_count[w];
+                count += warp_count[w];
+            }
+            if (first) {
+                rank[t] = at + __popc(b & ((1u << lane) - 1));
+                list[rank[t]] = t;
+            }
+            meet();
+        }
+        if (tid == 0) nlist = count;
+    } else if (warp == kBmFinders / 32) {
+        if (lane < 2 * np) {
+            const long long pr = p0 + lane / 2;
+            const int pt = (int)(pr % a.npointing), fi = (int)(pr / a.npointing);
+            const BmDir v = bm_dir2(lane & 1, np == 2 ? 0xFu : 0x3u, a.az[pt], a.za[pt], a.freq[fi]);
+            if ((lane & 1) == 0) dir[lane / 2] = v;
+        }
+    } else if (a.pa && lane < np) {
+        double p[4];
+        const int pt = (int)((p0 + lane) % a.npointing);
+        bm_pa(a.lat, a.az[pt], a.za[pt], p);
+        for (int e = 0; e < 4; e++) P[lane][e] = p[e];
     }
     __syncthreads();
-    // rep[t]: the first tile with tile t's delays; list: those first tiles
-    int count = 0;
-    for (int t0 = 0; t0 < a.ntile; t0 += kBmThreads) {
-        const int t = t0 + tid;
-        int r = t;
-        if (t < a.ntile) {
-            for (int u = 0; u < t; u++)
-                if (hash[u] == hash[t] && same_delays(a.delays, t, u)) {
-                    r = u;
-                    break;
-                }
-            rep[t] = r;
-        }
-        const bool first = t < a.ntile && r == t;
-        const unsigned b = __ballot_sync(0xffffffffu, first);
-        if (lane == 0) warp_count[warp] = __popc(b);
-        __syncthreads();
-        int at = count;
-        for (int w = 0; w < kBmThreads / 32; w++) {
-            if (w < warp) at += warp_count[w];
-            count += warp_count[w];
-        }
-        if (first) list[at + __popc(b & ((1u << lane) - 1))] = t;
-        __syncthreads();
-    }
+    const int share = blockIdx.y, shares = gridDim.y;
+    if (share >= nlist) return;
+    const int nsets = (nlist - share + shares - 1) / shares; // list[share + shares i]
 
-    if (a.pa && warp == kBmThreads / 32 - 1) {
-        if (lane < np) {
-            double p[4];
-            const int pt = (int)((p0 + lane) % a.npointing);
-            bm_pa(a.lat, a.az[pt], a.za[pt], p);
-            for (int e = 0; e < 4; e++) P[lane][e] = p[e];
-        }
-    }
     // items: (pair, set), 16 lanes each
-    const int groups = 2 * (kBmThreads / 32 - (a.pa ? 1 : 0)), group = tid >> 4, l = tid & 15;
-    const unsigned mask = 0xFFFFu << (lane & 16);
-    const int items = np * count;
+    const int items = np * nsets;
     double2 *out = a.B + 4 * p0 * a.ntile;
-    for (int e0 = 0; e0 < items; e0 += groups) {
-        const int e = e0 + group;
-        const bool mine = group < groups && e < items;
-        double2 J[4];
-        if (mine) {
-            const int pt = (int)((p0 + e / count) % a.npointing), fi = (int)((p0 + e / count) / a.npointing);
-            bm_jones16(l, mask, a.az[pt], a.za[pt], a.freq[fi], a.delays + 16 * (long long)list[e % count], J);
-        }
-        if (e0 == 0) __syncthreads(); // the rotations
-        if (mine && l == 0)
-            bm_store(out + 4 * ((long long)(e / count) * a.ntile + list[e % count]), J, a.pa ? P[e / count] : nullptr);
+    for (int e = tid >> 4; e < items; e += kBmGroups) {
+        const int j = e / nsets, t = list[share + shares * (e - j * nsets)];
+        bm_write16(tid & 15, 0xFFFFu << (lane & 16), dir[j], a.delays + 16 * (long long)t, a.pa ? P[j] : nullptr,
+                   out + 4 * ((long long)j * a.ntile + t));
     }
     __syncthreads();
-    // every other tile copies its set's matrix, 16 bytes per thread
+    // every other tile of these sets copies its set's matrix, 16 bytes per thread
     for (int i = tid; i < np * a.ntile * 4; i += kBmThreads) {
         const int t = (i / 4) % a.ntile, r = rep[t];
-        if (r != t) out[i] = out[i + 4 * (r - t)];
+        if (r != t && rank[r] % shares == share) out[i] = out[i + 4 * (r - t)];
     }
 }
 
@@ -249,9 +296,11 @@ int launch_beam_model(const PbArgs &a, cudaStream_t st, int *given)
     if (n <= 0) return VGB_SUCCESS;
     const long long pairs = (long long)a.nfreq * a.npointing;
     if (!given && a.ntile <= kBmMaxTiles && pairs <= kBmMaxPairs) {
-        const int per_block = pairs <= 152 ? 1 : 2; // one per SM, then two
-        beam_kernel_fused<<<(unsigned)((pairs + per_block - 1) / per_block), kBmThreads, 3 * sizeof(int) * a.ntile, st>>>(
-            a, per_block);
+        const int sms = sm_count(), per_block = pairs <= sms ? 1 : 2;
+        const int blocks = (int)((pairs + per_block - 1) / per_block);
+        // shares of the sets: down to one round of a block's lanes each, as long as each block has an SM to itself
+        const int shares = std::max(1, std::min((a.ntile + kBmGroups - 1) / kBmGroups, sms / blocks));
+        beam_kernel_fused<<<dim3(blocks, shares), kBmThreads, sizeof(int) * (bm_hashes(a.ntile) + 3 * a.ntile), st>>>(a, per_block);
         return check_launch("beam_kernel_fused");
     }
     int *scratch = given; // rep [ntile], list [ntile], count

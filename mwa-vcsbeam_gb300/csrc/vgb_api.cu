@@ -1,5 +1,6 @@
 // The plain C ABI (include/vcsbeam_gb300.h): argument checks, status
 // reporting and the one-second streaming pipeline.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -29,6 +30,20 @@ int check_cuda(cudaError_t e, const char *what)
 }
 
 int check_launch(const char *what) { return check_cuda(cudaGetLastError(), what); }
+
+// Asked once per device.
+int sm_count()
+{
+    static std::atomic<int> counts[64];
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && (n = counts[dev].load())) return n;
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        return 1;
+    }
+    if (dev >= 0 && dev < 64) counts[dev] = n;
+    return n;
+}
 
 // One status word per device, raised by kernels with atomicOr.
 __device__ unsigned g_status;

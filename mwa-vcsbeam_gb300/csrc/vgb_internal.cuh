@@ -64,6 +64,8 @@ struct VoltView {
 int set_error(int code, const char *fmt, ...);
 int check_cuda(cudaError_t e, const char *what);
 int check_launch(const char *what);
+// SMs of the current device.
+int sm_count();
 // Device address of the current device's status word (kernels atomicOr
 // kErr* bits into it), or NULL.
 unsigned *status_word();
