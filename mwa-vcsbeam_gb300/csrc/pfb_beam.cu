@@ -1476,11 +1476,15 @@ template <int A, bool B, bool C> struct PackSel {
         const size_t smem = std::max(least, base + sizeof(int) * (size_t)a.vv.ninputs);
         // Each CTA takes a share of the steps (the columns are independent), a
         // multiple of 4 (16 columns: the 4-bit mode's wide stores), so that the
-        // last wave is a small part: about 12 waves of CTAs, at least 8 steps
-        // each (a CTA's set-up costs about half a step).
-        const int nsteps = (a.vv.ninputs + kG - 1) / kG;
-        const long long want = 12LL * 456, ctas = (long long)grid.x * grid.y;
-        int parts = (int)std::min<long long>((want + ctas - 1) / ctas, std::max(1, nsteps / 8));
+        // last wave is a small part: about 36 CTAs per SM, at least 8 steps each
+        // (a CTA's set-up costs about half a step). Where those are less than a
+        // wave and a half of the places, 4 steps each: a run too short for the
+        // GPU takes a share's time (4 bits, 25 tiles, 300 spectra: 67 -> 28 us;
+        // 1,500: 118 -> 77; three channels of 1,500: 208 -> 200).
+        const int nsteps = (a.vv.ninputs + kG - 1) / kG, sms = sm_count();
+        const long long places = (C && A != kWolaSplit ? 3 : 2) * sms, want = 36LL * sms, ctas = (long long)grid.x * grid.y;
+        const int whole = std::max(1, nsteps / 8), most = 2 * ctas * whole < 3 * places ? (nsteps + 3) / 4 : whole;
+        const int parts = (int)std::min<long long>((want + ctas - 1) / ctas, most);
         PackArgs b = a;
         b.steps_per_cta = ((nsteps + parts - 1) / parts + 3) / 4 * 4;
         grid.z = (nsteps + b.steps_per_cta - 1) / b.steps_per_cta;
