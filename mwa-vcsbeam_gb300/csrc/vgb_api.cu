@@ -891,8 +891,16 @@ int vgb_pipeline_set_filters(vgb_pipeline *p, const int32_t *analysis, const flo
 {
     if (!p || !analysis) return set_error(VGB_ERR_INVALID, "NULL argument");
     if (p->cfg.do_ipfb && !synthesis) return set_error(VGB_ERR_INVALID, "synthesis filter required for the IPFB");
+    int rc = check_cuda(cudaStreamSynchronize(p->s_comp), "sync");
+    if (rc) return rc;
+    const unsigned before = pipeline_pfb_flags(p);
     p->wola_flags = vgb_filter_wola_flags(analysis, kP, kK);
-    int rc = check_cuda(cudaMemcpyAsync(p->d_filter, analysis, sizeof(int32_t) * kK * kP, cudaMemcpyHostToDevice,
+    if (pipeline_pfb_flags(p) != before) {
+        // the captured seconds and the timed kernel variant are another overlap-add's
+        drop_graphs(p);
+        p->front_timed = false;
+    }
+    rc = check_cuda(cudaMemcpyAsync(p->d_filter, analysis, sizeof(int32_t) * kK * kP, cudaMemcpyHostToDevice,
                                         p->s_comp),
                         "upload analysis filter");
     if (!rc && synthesis)
