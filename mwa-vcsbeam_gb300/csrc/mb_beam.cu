@@ -26,9 +26,9 @@
 //   R[(p, st)](t) = sum_{a, j} Q[(p, st), (a, j)] Cint[(a, j)](t),
 // j in {C_QQ, C_PP, Re C_QP, Im C_QP}, st the Stokes parameter. It runs on the
 // FP16 tensor path (tc_gemm.cu): integrated coherencies of 4-bit voltages are
-// exact in FP16, those of 8-bit voltages are split into exact hi + lo halves,
-// and Q carries a power-of-two scale per row (and, in the split mode, an FP16
-// lo half).
+// exact in FP16, those of 8-bit voltages are split into exact hi + lo halves of
+// an eighth of them (ten samples of full range reach 327,680, FP16 65,504), and Q
+// carries a power-of-two scale per row (and, in the split mode, an FP16 lo half).
 //
 // The beam GEMM's epilogue reads the accumulators back with tcgen05.ld,
 // forms XX, YY, XY per sample across the four lanes that hold one beam,
@@ -58,6 +58,8 @@ constexpr int kMbUsed = 250;   // samples of a tile that are used: 25 integratio
 constexpr int kMbNint = kMbUsed / kMbInt;
 constexpr int kMbBeamsPerTile = 32;  // 128 rows / 4
 constexpr int kMbEpq = 3;            // epilogue warps per TMEM lane quarter
+constexpr int kMbCohExp = 3;         // 8-bit coherencies are stored times 2^-kMbCohExp
+constexpr float kMbCohScale = 1 << kMbCohExp;
 constexpr int kMbEpiWarps = 4 * kMbEpq;
 constexpr int kMbThreads = 64 + 32 * kMbEpiWarps; // warp 0 TMA, warp 1 MMA, warps 2.. epilogue
 constexpr uint32_t kMbPolls = 1u << 26;
@@ -319,7 +321,7 @@ __device__ __forceinline__ void mb_q_scales(const MbWeightArgs &w, int c, int p,
         int e = 0;
         if (m > 0.f && isfinite(m)) frexpf(m, &e); // m = f 2^e, f in [0.5, 1)
         inv_scale[st] = ldexpf(1.f, -e);
-        if (threadIdx.x == 0 && st < w.nst) w.qscale[(long long)c * w.Mq + p * w.nst + st] = ldexpf(1.f, e);
+        if (threadIdx.x == 0 && st < w.nst) w.qscale[(long long)c * w.Mq + p * w.nst + st] = ldexpf(1.f, w.int8 ? e + kMbCohExp : e);
     }
 }
 
@@ -489,7 +491,8 @@ __global__ void __launch_bounds__(256, 4) mb_weights_pair_kernel(const MbWeightA
 // ---------------------------------------------------------------------------
 // Voltages: legacy [s][c][input] (4+4-bit bytes, high nibble real, or int8
 // re, im) -> B operand V [c][s][4A] (bf16 or fp16, exact) and the integrated
-// per-tile coherencies C [c][t][Kb] (fp16; exact hi/lo halves for 8-bit).
+// per-tile coherencies C [c][t][Kb] (fp16; exact hi/lo halves of an eighth for
+// 8-bit, which the row scales or the FP32 reader give back).
 // ---------------------------------------------------------------------------
 struct MbConvArgs {
     const uint8_t *v;
@@ -553,9 +556,10 @@ __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
         const int cv[4] = {cqq, cpp, cr, ci};
         uint16_t hi[4], lo[4];
         for (int j = 0; j < 4; j++) {
-            const __half h = __float2half_rn((float)cv[j]);
+            const float cf = g.int8 ? (float)cv[j] * (1.f / kMbCohScale) : (float)cv[j];
+            const __half h = __float2half_rn(cf);
             hi[j] = __half_as_ushort(h);
-            lo[j] = __half_as_ushort(__float2half_rn((float)(cv[j] - (int)__half2float(h))));
+            lo[j] = __half_as_ushort(__float2half_rn(cf - __half2float(h)));
         }
         __half *row = g.C + ((long long)c * g.nint_p + t) * g.Kb;
         *reinterpret_cast<uint2 *>(row + 4 * a) =
@@ -636,9 +640,10 @@ template <bool kInt8> __global__ void __launch_bounds__(128) mb_gather_voltages_
             const int cv[4] = {cqq[j] >> kShift, cpp[j] >> kShift, cr[j] >> kShift, (cqp[j] - cpq[j]) >> kShift};
             uint16_t hi[4], lo[4];
             for (int i = 0; i < 4; i++) {
-                const __half h = __float2half_rn((float)cv[i]);
+                const float cf = (float)cv[i] * (kInt8 ? 1.f / kMbCohScale : 1.f);
+                const __half h = __float2half_rn(cf);
                 hi[i] = __half_as_ushort(h);
-                lo[i] = __half_as_ushort(__float2half_rn((float)(cv[i] - (int)__half2float(h))));
+                lo[i] = __half_as_ushort(__float2half_rn(cf - __half2float(h)));
             }
             __half *row = g.C + ((long long)c * g.nint_p + t) * g.Kb + 4 * (kT * u + j);
             *reinterpret_cast<uint2 *>(row) = make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
@@ -1563,7 +1568,7 @@ __global__ void __launch_bounds__(256) mb_simt_auto_kernel(const MbSimtAutoArgs 
             if (t < g.nint) {
                 const __half *row = g.C + ((long long)c * g.nint_p + t) * g.Kb;
                 cv = __half2float(row[k0 + k]);
-                if (g.int8) cv += __half2float(row[g.KA + k0 + k]);
+                if (g.int8) cv = kMbCohScale * (cv + __half2float(row[g.KA + k0 + k]));
             }
             Cs[k][i] = cv;
         }
