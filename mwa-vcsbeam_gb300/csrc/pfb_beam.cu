@@ -1345,17 +1345,7 @@ static std::atomic<int> g_pfb_last{0};    // inputs per step of the last fused l
 // the spectra of a leftover tile.
 static int beam_tiles(BeamArgs &a, int ncc, int per_sm, int least, int step)
 {
-    static std::atomic<int> sms{0};
-    if (!sms.load()) {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-            n <= 0) {
-            cudaGetLastError();
-            n = 152;
-        }
-        sms = n;
-    }
-    const long long slots = (long long)per_sm * sms.load(), total = (long long)a.nspectra * ncc;
+    const long long slots = (long long)per_sm * sm_count(), total = (long long)a.nspectra * ncc;
     a.ncc = ncc;
     const long long full = total / (kT * slots) * slots; // tiles in whole waves
     const int n8 = (int)std::min<long long>(full / ncc, a.nspectra / kT);

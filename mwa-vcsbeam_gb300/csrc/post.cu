@@ -541,9 +541,9 @@ template <int kCh, bool kStats> static int launch_renorm4(const RenormArgs &a, i
 {
     auto kern = renorm4_kernel<kCh, kStats>;
     cudaLaunchConfig_t cfg = {};
-    // with the extremes given: enough blocks for four per SM
+    // with the extremes given: about eight blocks per SM
     const long long groups = (long long)(a.nchan / kCh) * a.npointing * a.nstokes * ncc;
-    const long long parts = kStats ? std::max(1LL, std::min<long long>(a.nstep / 256 + 1, (8 * 152 + groups - 1) / groups))
+    const long long parts = kStats ? std::max(1LL, std::min<long long>(a.nstep / 256 + 1, (8 * sm_count() + groups - 1) / groups))
                                    : kRenormSplit;
     cfg.gridDim = dim3((unsigned)(parts * (a.nchan / kCh)), a.npointing * a.nstokes, ncc);
     cfg.blockDim = dim3(256);
@@ -1217,9 +1217,7 @@ int launch_legacy_beam(const LegacyArgs &a, cudaStream_t st)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: %d inputs do not fit the shared-memory tile", ni);
     if ((a.nsamples + kLS - 1) / kLS > 65535)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: at most %d samples per call", 65535 * kLS);
-    int nsm = 1, dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-        return check_cuda(cudaGetLastError(), "cudaDeviceGetAttribute(legacy)");
+    const int nsm = sm_count();
     const LegacyTile t = legacy_tile(a, int4, nsm);
     const long long blocks = (long long)((a.nchan + t.channels - 1) / t.channels) * ((a.nsamples + t.samples - 1) / t.samples);
     if (t.smem <= 227 * 1024 && blocks <= INT_MAX) {
