@@ -11,7 +11,6 @@
 //    (v_IDX [s][c][i], 4+4-bit or complex FP64): vmApplyJ_kernel followed by
 //    vmBeamform_kernel (form_beam.cpp:122-371) in one pass.
 #include <algorithm>
-#include <climits>
 #include <type_traits>
 
 #include <cooperative_groups.h>
@@ -651,6 +650,8 @@ int launch_incoh(const uint8_t *data, long long nrows, int ninput, float *incoh,
 // complex doubles: 1,440 -> 282 us (shared-memory pipe 60-70 %, the FP64
 // voltages read once instead of once per beam).
 
+constexpr int kLS = 4; // samples of a row kernel's block: a call takes 65,535 times as many
+
 // The 8 sums of a pair of samples over a tile: a[0..3] += ex, ey (re, im);
 // a[4..7] += |ex|^2, |ey|^2, ex ey* (re, im). w: the two Jones rows with each
 // value doubled into a pair; nw: minus the imaginary parts of w.
@@ -700,15 +701,6 @@ __device__ __forceinline__ void legacy_store(const LegacyArgs &a, int p, int s, 
     if (a.e) a.e[((long long)p * a.nsamples + s) * a.nchan + c] = make_float4(acc[0], acc[1], acc[2], acc[3]);
 }
 
-// Tiles of channels and samples on grid x, channels fastest: two samples a tile
-// make more sample tiles than grid y counts (65,535) well within a call's limit.
-template <int kCh, int kSamp> __device__ __forceinline__ void legacy_origin(const LegacyArgs &a, int &c0, int &s0)
-{
-    const unsigned across = (unsigned)(a.nchan + kCh - 1) / kCh;
-    c0 = (int)(blockIdx.x % across) * kCh;
-    s0 = (int)(blockIdx.x / across) * kSamp;
-}
-
 // The tiles' (Q, P) input pairs into shared memory, checked against the row.
 __device__ __forceinline__ void legacy_inputs(const LegacyArgs &a, uint32_t *pq)
 {
@@ -716,7 +708,7 @@ __device__ __forceinline__ void legacy_inputs(const LegacyArgs &a, uint32_t *pq)
     for (int ant = threadIdx.x; ant < a.nant; ant += blockDim.x) {
         uint32_t iq = __ldg(a.polQ + ant), ip = __ldg(a.polP + ant);
         if (iq >= ni || ip >= ni) {
-            if (blockIdx.x == 0) atomicOr(a.status, kErrBadInput);
+            if (blockIdx.x == 0 && blockIdx.y == 0) atomicOr(a.status, kErrBadInput);
             iq = ip = 0;
         }
         pq[ant] = iq | (ip << 16);
@@ -766,8 +758,7 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 2) legacy4_kern
     Word *vt = reinterpret_cast<Word *>(red + kL4Red);
     uint32_t *pq = reinterpret_cast<uint32_t *>(vt + (size_t)kG * ni * kL4C);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int c0, s0;
-    legacy_origin<kL4C, kS * kG>(a, c0, s0);
+    const int c0 = blockIdx.x * kL4C, s0 = blockIdx.y * kS * kG;
 
     legacy_inputs(a, pq);
     // stage: lane = (channel 4 warp + lane % 4, word lane / 4 of 8), so 8 lanes
@@ -924,8 +915,7 @@ template <int kS, int kG> __global__ void __launch_bounds__(256, 3) legacyd_kern
     float *red = reinterpret_cast<float *>(vt + (size_t)kPairs * kG * kLdC * stride); // partial sums
     uint32_t *pq = reinterpret_cast<uint32_t *>(red + kLWarps * kS * 8 * kLdC);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    int c0, s0;
-    legacy_origin<kLdC, kS * kG>(a, c0, s0);
+    const int c0 = blockIdx.x * kLdC, s0 = blockIdx.y * kS * kG + (kS * kG < kLS ? a.s_first : 0);
 
     legacy_inputs(a, pq);
     // warp w stages channel w's rows, two sample pairs in flight
@@ -1094,7 +1084,7 @@ static LegacyTile legacy_tile(const LegacyArgs &a, bool int4, int nsm)
 // 4-byte pad (33 KB for 256 tiles, so several blocks share an SM).
 // ---------------------------------------------------------------------------
 
-constexpr int kLS = 4, kLC = 16; // samples, channels per block
+constexpr int kLC = 16;          // channels per block
 constexpr int kLParts = 4;       // threads per row
 
 template <bool kInt4>
@@ -1219,16 +1209,23 @@ int launch_legacy_beam(const LegacyArgs &a, cudaStream_t st)
         return set_error(VGB_ERR_INVALID, "legacy beamformer: at most %d samples per call", 65535 * kLS);
     const int nsm = sm_count();
     const LegacyTile t = legacy_tile(a, int4, nsm);
-    const long long blocks = (long long)((a.nchan + t.channels - 1) / t.channels) * ((a.nsamples + t.samples - 1) / t.samples);
-    if (t.smem <= 227 * 1024 && blocks <= INT_MAX) {
+    if (t.smem <= 227 * 1024) {
         const int rc = check_cuda(cudaFuncSetAttribute(t.kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)t.smem),
                                   "cudaFuncSetAttribute(legacy tile)");
         if (rc) return rc;
+        const unsigned gx = (a.nchan + t.channels - 1) / t.channels, gy = (a.nsamples + t.samples - 1) / t.samples;
         // the pointings over blocks too where the rest is short of two (4-bit) or one (FP64) per SM: each
         // share reads the voltages again (4-bit, 20 tiles, 200 samples, 12 beams: 74 -> 21 us)
-        const long long shares = (int4 ? 2 : 1) * nsm / blocks;
+        const long long shares = (int4 ? 2 : 1) * nsm / ((long long)gx * gy);
         const unsigned gz = (unsigned)std::min<long long>(a.npointing, std::max<long long>(1, shares));
-        t.kern<<<dim3((unsigned)blocks, 1, gz), 256, t.smem, st>>>(a);
+        // grid y counts 65,535 tiles of samples; those of two (FP64, 208 to 877 tiles) can be twice as many
+        // and come in two launches. (A first sample in the other kernels too, or both directions on grid x
+        // with a division a block: 4-bit 252 -> 256 us.)
+        LegacyArgs part = a;
+        for (unsigned y = 0; y < gy; y += 65535) {
+            part.s_first = (int)y * t.samples;
+            t.kern<<<dim3(gx, std::min(gy - y, 65535u), gz), 256, t.smem, st>>>(part);
+        }
         return check_launch("legacy beam kernel");
     }
     dim3 grid((a.nchan + kLC - 1) / kLC, (a.nsamples + kLS - 1) / kLS);

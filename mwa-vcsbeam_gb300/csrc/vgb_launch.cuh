@@ -77,6 +77,7 @@ struct LegacyArgs {
     float4 *e;               // [p][s][nchan] nullable
     float *incoh;            // [s][nchan] nullable (int4 only)
     unsigned *status;        // kErrBadInput when polQ / polP name an input outside the row
+    int s_first;             // set by the launcher: the launch's first sample (tiles of two samples)
 };
 
 struct IpfbArgs {
