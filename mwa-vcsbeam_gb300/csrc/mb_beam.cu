@@ -496,7 +496,6 @@ __global__ void __launch_bounds__(256, 4) mb_weights_pair_kernel(const MbWeightA
 // ---------------------------------------------------------------------------
 struct MbConvArgs {
     const uint8_t *v;
-    int int8, fp16;
     int ns, nfine, ni, A, nint, nint_p, Kb;
     const uint32_t *polQ, *polP;
     unsigned *status;     // kErrBadInput when polQ / polP name an input outside the row
@@ -509,14 +508,15 @@ __device__ __forceinline__ int nib4(uint32_t x) { return ((int)(x << 28)) >> 28;
 // One block per (channel, integration), channels fastest so that neighbouring
 // blocks read neighbouring bytes of each sample: the 10 voltage rows (2A
 // inputs each) are staged in shared memory with 16-byte loads, then each
-// thread gathers its tiles' (Q, P) inputs through polQ/polP.
-__global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
+// thread gathers its tiles' (Q, P) inputs through polQ/polP. Bound by memory;
+// one kernel per input and operand type (256 tiles of 4-bit voltages, 10^4 samples:
+// 0.53 ms; with both tested inside 0.70 since the 8-bit coherencies are scaled).
+template <bool kInt8, bool kF16> __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
 {
     extern __shared__ uint4 conv_smem[];
     uint8_t *rows = reinterpret_cast<uint8_t *>(conv_smem);
     const int c = blockIdx.x, t = blockIdx.y;
-    const bool h16 = g.fp16 != 0;
-    const int rowbytes = g.ni * (g.int8 ? 2 : 1); // a multiple of 32 (nant % 16 == 0)
+    const int rowbytes = g.ni * (kInt8 ? 2 : 1); // a multiple of 32 (nant % 16 == 0)
     const int per_row = rowbytes / 16;
     // all of the block's row loads in flight at once (asynchronous copies), one wait
     for (int e = threadIdx.x; e < kMbInt * per_row; e += blockDim.x) {
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
             const int s = t * kMbInt + k;
             const uint8_t *r = rows + k * rowbytes;
             int qr, qi, pr, pi;
-            if (g.int8) {
+            if (kInt8) {
                 const char2 vq = reinterpret_cast<const char2 *>(r)[iq];
                 const char2 vp = reinterpret_cast<const char2 *>(r)[ip];
                 qr = vq.x; qi = vq.y; pr = vp.x; pi = vp.y;
@@ -549,14 +549,14 @@ __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
             cpp += pr * pr + pi * pi;
             cr += qr * pr + qi * pi; // Re(vQ vP*)
             ci += qi * pr - qr * pi; // Im(vQ vP*)
-            const uint2 o = make_uint2(to_bits((float)qr, h16) | ((uint32_t)to_bits((float)qi, h16) << 16),
-                                       to_bits((float)pr, h16) | ((uint32_t)to_bits((float)pi, h16) << 16));
+            const uint2 o = make_uint2(to_bits((float)qr, kF16) | ((uint32_t)to_bits((float)qi, kF16) << 16),
+                                       to_bits((float)pr, kF16) | ((uint32_t)to_bits((float)pi, kF16) << 16));
             *reinterpret_cast<uint2 *>(g.V + ((long long)c * g.ns + s) * (4 * g.A) + 4 * a) = o;
         }
         const int cv[4] = {cqq, cpp, cr, ci};
         uint16_t hi[4], lo[4];
         for (int j = 0; j < 4; j++) {
-            const float cf = g.int8 ? (float)cv[j] * (1.f / kMbCohScale) : (float)cv[j];
+            const float cf = (float)cv[j] * (kInt8 ? 1.f / kMbCohScale : 1.f);
             const __half h = __float2half_rn(cf);
             hi[j] = __half_as_ushort(h);
             lo[j] = __half_as_ushort(__float2half_rn(cf - __half2float(h)));
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(128) mb_convert_kernel(const MbConvArgs g)
         __half *row = g.C + ((long long)c * g.nint_p + t) * g.Kb;
         *reinterpret_cast<uint2 *>(row + 4 * a) =
             make_uint2(hi[0] | ((uint32_t)hi[1] << 16), hi[2] | ((uint32_t)hi[3] << 16));
-        if (g.int8)
+        if (kInt8)
             *reinterpret_cast<uint2 *>(row + 4 * g.A + 4 * a) =
                 make_uint2(lo[0] | ((uint32_t)lo[1] << 16), lo[2] | ((uint32_t)lo[3] << 16));
     }
@@ -2126,8 +2126,6 @@ int mb_run_cc(vgb_multibeam *mb, int cc, const uint8_t *v_cc, float *S_cc, uint8
 
     MbConvArgs g{};
     g.v = v_cc;
-    g.int8 = mb->int8;
-    g.fp16 = mb->fp16;
     g.ns = ns;
     g.nfine = nf;
     g.ni = 2 * A;
@@ -2141,7 +2139,9 @@ int mb_run_cc(vgb_multibeam *mb, int cc, const uint8_t *v_cc, float *S_cc, uint8
     g.V = mb->d_V;
     g.C = mb->d_C;
     const int conv_smem = kMbInt * 2 * A * (mb->int8 ? 2 : 1);
-    auto conv = !mb->few ? mb_convert_kernel : mb->int8 ? mb_gather_voltages_kernel<true> : mb_gather_voltages_kernel<false>;
+    auto conv = mb->few ? (mb->int8 ? mb_gather_voltages_kernel<true> : mb_gather_voltages_kernel<false>)
+                : mb->int8 ? (mb->fp16 ? mb_convert_kernel<true, true> : mb_convert_kernel<true, false>)
+                           : (mb->fp16 ? mb_convert_kernel<false, true> : mb_convert_kernel<false, false>);
     const int conv_threads = mb->few && !mb->int8 && A <= 128 ? 64 : 128;
     if ((rc = check_cuda(cudaFuncSetAttribute(conv, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem),
                          "cudaFuncSetAttribute(mb_convert_kernel)")))
