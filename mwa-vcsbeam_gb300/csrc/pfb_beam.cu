@@ -795,12 +795,12 @@ __device__ __forceinline__ void beam_tm_body(const BeamArgs &a, const CUtensorMa
         // step it's frames have landed and every thread has finished step it - 1
         const bool got = mbar_wait_bounded(&sm.bar_f[it % kStages], it / kStages & 1, 1u << 22);
         if (__syncthreads_or(!got || wbad)) break;
-        if (it > 0) tm_weights(sm, wmap, cc, it);
-        if (kStages == 2 && it + 1 < nsteps) tm_frames<T>(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
-        __syncwarp(); // lane 0 has copied
         {
             typename WolaTap<kW>::type t[kP];
-            tm_taps<kW>(ttab, t);
+            tm_taps<kW>(ttab, t); // warp-collective: before lane 0 copies
+            if (it > 0) tm_weights(sm, wmap, cc, it);
+            if (kStages == 2 && it + 1 < nsteps) tm_frames<T>(sm, a.vv, cc, it + 1, m0, a.nspectra, a.status);
+            __syncwarp();
             wola_rows<kW, kFpga, T, kTmPass>(sm.stage[it % kStages][li][0], &sm.buf[li * kT], n0, t);
         }
         input_barrier(li);
