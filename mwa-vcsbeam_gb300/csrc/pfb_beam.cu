@@ -703,7 +703,7 @@ static_assert(offsetof(TmSmem<1>, wst) % 128 == 0 && offsetof(TmSmem<1>, buf) % 
 // at 0 and 36, their tables at 72
 constexpr uint32_t kTmCols = 128, kTmTables = 72;
 
-// Frames of step `it` into the single stage: lane 0 of warp li (li < kG)
+// Frames of step `it` into stage it % kStages: lane 0 of warp li (li < kG)
 // copies input it * kG + li, lane 0 of warp 0 posts the byte count first
 // (completing its own shortfall when frames fell outside the buffers, as
 // produce_spread does).
@@ -1142,12 +1142,13 @@ __device__ __forceinline__ void pack_frames(PackSmem &sm, const VoltView &vv, in
 
 // The beam kernels' front end at three CTAs per SM (tables from tensor memory,
 // frames single-buffered and copied while the step's rows are written out, at
-// most 80 registers; the split sums need 122, two CTAs) and the packing of its
-// rows. kDemote is the 4-bit output. Against two CTAs per SM with taps and
-// held words in registers, every column in one CTA and the instruction's
-// conversions: 10,000 spectra x 256 inputs to 4 bits with int32 sums 1,353 ->
-// 1,060 us (issue 70 %, FMA and ALU pipes 42 %), 4,000 spectra to complex
-// double 787 -> 565 us (shared-memory pipe 65 %, DRAM 50 %: 3.7 TB/s written).
+// most 80 registers) and the packing of its rows. kDemote is the 4-bit output.
+// Two CTAs per SM for the split sums (122 registers) and for complex doubles
+// (the launcher asks for the shared memory: fewer rows open). Against two with
+// taps and held words in registers, every column in one CTA and the
+// instruction's conversions: 10,000 spectra x 256 inputs to 4 bits with int32
+// sums 1,353 -> 1,060 us (issue 69 %, FMA and ALU pipes 37 and 44 %), 4,000
+// spectra to complex double 787 -> 556 us (shared-memory pipe 56 %, DRAM 52 %).
 template <int kW, bool kFpga, bool kDemote>
 __global__ void __launch_bounds__(kThreads, kW == kWolaSplit ? 2 : 3) pack_kernel(const PackArgs a)
 {

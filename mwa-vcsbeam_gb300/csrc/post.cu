@@ -649,9 +649,9 @@ int launch_incoh(const uint8_t *data, long long nrows, int ninput, float *incoh,
 // than per sample. Sums are kept for pairs of samples in FP32x2, so one issue
 // slot covers two multiply-adds and half of the slots are left for the loads
 // and the widening of the voltages. One beam of 128 tiles x 128 channels x
-// 10,000 samples of 4+4-bit voltages: 1,060 -> 257 us against the row kernel
-// below (FMA pipe 59 % busy, issue 63 %); three beams of 2,000 samples of
-// complex doubles: 1,440 -> 282 us (shared-memory pipe 60-70 %, the FP64
+// 10,000 samples of 4+4-bit voltages: 1,060 -> 252 us against the row kernel
+// below (issue 63 %, ALU pipe 50 %); three beams of 2,000 samples of complex
+// doubles: 1,440 -> 283 us (shared-memory pipe 57 %, DRAM 47 %, the FP64
 // voltages read once instead of once per beam).
 
 constexpr int kLS = 4; // samples of a row kernel's block: a call takes 65,535 times as many
